@@ -16,7 +16,6 @@ discipline and error behaviour, so model code written against it runs unchanged.
 One process per GPU runs the same program; every reduction returns bitwise-identical values on all ranks.
 """
 
-import ctypes as C
 import os
 
 import torch
@@ -107,6 +106,8 @@ class Group:
         self._buffers = {}
         self._handles = {}
         self._recv = {}
+        self._by_address = {}  # base address of a symmetric buffer -> its key
+        self._calls = {}       # (site, chain, rows, n, mode, one hop) -> (DlmComm template, output buffer)
         self._out_peers = {}
         self._last = {}      # per chain: the previous call's output buffer
         self._pending = {}   # partial data_ptr -> (linear, x): GEMMs deferred into the next reduction
@@ -131,19 +132,31 @@ class Group:
         reach the buffer.
         """
         if key not in self._buffers:
-            self._buffers[key], self._handles[key] = self._alloc.alloc(tuple(shape), dtype, armed)
+            t, self._handles[key] = self._alloc.alloc(tuple(shape), dtype, armed)
+            self._buffers[key] = t
+            self._by_address[t.data_ptr()] = key
         t = self._buffers[key]
-        if tuple(t.shape) != tuple(shape) or t.dtype != dtype:  # never hand out a view the caller may overrun
+        if t.shape != tuple(shape) or t.dtype != dtype:  # never hand out a view the caller may overrun
             raise ValueError(f"symmetric buffer {key}: {tuple(t.shape)} {t.dtype} allocated, {tuple(shape)} {dtype} "
                              "requested")
         return t
 
+    def _key(self, t):
+        """The key of the symmetric buffer that `t` is (a view of), or None."""
+        address = t.data_ptr()
+        key = self._by_address.get(address)
+        if key is None:  # not a buffer's first element: look for the buffer it lies in
+            for name, buf in self._buffers.items():
+                base = buf.data_ptr()
+                if base <= address < base + buf.numel() * buf.element_size():
+                    return name
+        return key
+
     def _handle(self, t):
-        for key, buf in self._buffers.items():
-            base = buf.data_ptr()
-            if base <= t.data_ptr() < base + buf.numel() * buf.element_size():
-                return key, self._handles[key]
-        raise ValueError("not a symmetric tensor of this group")
+        key = self._key(t)
+        if key is None:
+            raise ValueError("not a symmetric tensor of this group")
+        return key, self._handles[key]
 
     def multicast(self, t):
         """The NVSwitch multicast address that aliases `t` on all ranks at once (one store lands in every copy);
@@ -196,11 +209,7 @@ class Group:
     def is_partial(self, t):
         """True when `t` is (a leading-rows view of) this group's symmetric memory, i.e. a GEMM into it may be fused
         into the reduction that follows."""
-        try:
-            self._handle(t)
-        except ValueError:
-            return False
-        return True
+        return self._key(t) is not None
 
     def defer(self, linear, x, out):
         """Record `out = x @ linear.weight^T` instead of running it; the next reduce* of `out` runs it fused."""
@@ -208,8 +217,12 @@ class Group:
         return out
 
     def defer_experts(self, out, down):
-        """Record the NVFP4 expert down-projection + combine into `out` (keyword arguments of
-        dlmrt_b200.quantization.nvfp4.moe_down) instead of running it; the next reduce* of `out` runs it fused."""
+        """Record the NVFP4 expert down-projection + combine into `out` (a dlmrt_b200.quantization.nvfp4.Down, or keyword
+        arguments of its moe_down) instead of running it; the next reduce* of `out` runs it fused."""
+        from ..quantization import nvfp4
+
+        if not isinstance(down, nvfp4.Down):
+            down = nvfp4.Down(nvfp4.descriptor(**down), down)
         self._pending[out.data_ptr()] = ("experts", down, None, out)
         return out
 
@@ -220,7 +233,7 @@ class Group:
         else:
             from ..quantization import nvfp4
 
-            nvfp4.moe_down(out=out, **what)
+            nvfp4._run_down(what.m, out)
 
     def flush(self, partial):
         """Run a deferred producer on its own, for callers that read the partial before reducing it."""
@@ -239,61 +252,73 @@ class Group:
         return ws
 
     # -- launches ---------------------------------------------------------------------------------------------------
+    def _call(self, rows, n, site, chain, mode, one_shot):
+        """What every call at one site has in common (the bookkeeping of parallel.py:119-132): a DlmComm with the
+        buffers' addresses filled in, and the output buffer. Made once; a call copies it and sets what it brings."""
+        key = site, chain, rows, n, mode, one_shot
+        call = self._calls.get(key)
+        if call is None:
+            out = self.symmetric(f"out:{site}", (rows, n), armed=True)
+            ptrs, epochs, recv_mc = self._receive(rows, n, chain, one_shot)
+            c = DlmComm()
+            c.rank, c.world, c.rows, c.n, c.mode = self.rank, self.world, rows, n, mode
+            peers = self.peer_addresses(out)
+            for s in range(self.world):
+                c.recv[s] = ptrs[s]
+                c.out_peers[s] = peers[s]
+            c.out = out.data_ptr()
+            c.out_mc = self.multicast(out) or None
+            c.epochs = epochs.data_ptr()
+            c.status = self.status.data_ptr()
+            c.one_shot, c.recv_mc = int(one_shot), (recv_mc or None) if one_shot else None
+            call = self._calls[key] = c, out
+        return call
+
     def _comm(self, rows, n, site, chain, mode, h, weight, eps, scale, replicated=False):
-        """The DlmComm of one call and its output buffer (the bookkeeping of parallel.py:119-132)."""
-        out = self.symmetric(f"out:{site}", (rows, n), armed=True)
+        """The DlmComm of one call and its output buffer."""
         # A replicated residual stream needs every row on every rank: always one hop, whatever the size.
-        one_shot = self.one_shot(rows, n, mode) or (replicated and self.world > 1)
-        ptrs, epochs, recv_mc = self._receive(rows, n, chain, one_shot)
+        one_shot = self.world > 1 and (replicated or self.one_shot(rows, n, mode))
+        template, out = self._call(rows, n, site, chain, mode, one_shot)
         last = self._last.get(chain)
         if last is out:  # same wording as parallel.py:124-125: callers may match on it
             raise ValueError(f"call site {site} ran twice in a row; its buffer would never be re-armed")
-        c = DlmComm()
-        c.rank, c.world, c.rows, c.n, c.mode = self.rank, self.world, rows, n, mode
+        c = DlmComm.from_buffer_copy(template)
         c.eps, c.scale = eps, scale
-        peers = self.peer_addresses(out)
-        for s in range(self.world):
-            c.recv[s] = ptrs[s]
-            c.out_peers[s] = peers[s]
-        c.out = out.data_ptr()
-        c.out_mc = self.multicast(out) or None
         # Whatever this chain produced last has been consumed by now: this launch resets it to "not arrived".
         if last is not None:
-            c.rearm, c.rearm_bytes = last.data_ptr(), last.numel() * last.element_size()
-        c.epochs = epochs.data_ptr()
-        c.h = h.data_ptr() if h is not None else None
-        c.weight = weight.data_ptr() if weight is not None else None
-        c.status = self.status.data_ptr()
+            c.rearm, c.rearm_bytes = last.data_ptr(), last.nbytes
+        if h is not None:
+            c.h = h.data_ptr()
+        if weight is not None:
+            c.weight = weight.data_ptr()
         c.stamps = self.stamps or None
         c.timeout_ns = TIMEOUT_NS
-        c.pdl = int(PDL)
+        c.pdl = PDL
         c.max_ctas = self.max_ctas
-        c.one_shot, c.recv_mc = int(one_shot), (recv_mc or None) if one_shot else None
         return c, out
 
     def _gemm(self, linear, x, chain):
-        g = DlmGemm()
         m, k = x.shape
-        if x.stride(1) != 1 or x.dtype != torch.bfloat16:
+        ldx, step = x.stride()
+        if step != 1 or x.dtype != torch.bfloat16:
             raise ValueError("row-parallel input must be BF16 with contiguous K")
-        nbytes = _lib.lib().dlm_workspace_bytes(m, linear.n, k)
+        template, nbytes = linear.plan(m)
         ws = self.workspace(chain, nbytes)
+        g = DlmGemm.from_buffer_copy(template)
         linear.describe(g)
-        g.x, g.m, g.n, g.k, g.ldx = x.data_ptr(), m, linear.n, k, x.stride(0)
+        g.x, g.k, g.ldx = x.data_ptr(), k, ldx
         g.workspace, g.workspace_bytes = ws.data_ptr(), ws.numel()
         g.splits, g.token_tiles = linear.splits, linear.token_tiles
         return g
 
     @staticmethod
-    def _overlap(a, b):
-        """Whether tensors a and b share any byte (by address range)."""
-        if a is None or b is None:
+    def _overlap(x, other):
+        """Whether a GEMM input [m, k] and a contiguous buffer share any byte (by address range)."""
+        if x is None or other is None:
             return False
-        a0, b0 = a.data_ptr(), b.data_ptr()
-        a1 = a0 + ((a.shape[0] - 1) * a.stride(0) + a.shape[1]) * a.element_size() if a.dim() == 2 else \
-            a0 + a.numel() * a.element_size()
-        b1 = b0 + b.numel() * b.element_size()
-        return a0 < b1 and b0 < a1
+        x0, o0 = x.data_ptr(), other.data_ptr()
+        m, k = x.shape
+        return x0 < o0 + other.nbytes and o0 < x0 + ((m - 1) * x.stride(0) + k) * 2
 
     def _launch(self, mode, partial, h, weight, site, eps=0.0, scale=1.0, chain=0, replicated=False):
         if self._failed:
@@ -302,27 +327,25 @@ class Group:
         rows, n = partial.shape
         last = self._last.get(chain)
         comm, out = self._comm(rows, n, site, chain, mode, h, weight, eps, scale, replicated)
-        stream = torch.cuda.current_stream(self.device).cuda_stream
-        pending = self._pending.pop(partial.data_ptr(), None)
+        stream = _lib.stream(self.status)
+        address = partial.data_ptr()
+        pending = self._pending.pop(address, None)
+        lib = _lib.lib()
         # The fused kernel re-arms `last` and fills `out` while other CTAs still load the GEMM's input; an input that
         # IS one of those (a projection fed straight from the previous reduction) therefore runs as two kernels, the
         # order the reference has anyway.
         fusable = pending is not None and n <= _lib.FUSED_MAX_N and not self._overlap(pending[2], last) \
             and not self._overlap(pending[2], out)
         if fusable and pending[0] == "linear":
-            gemm = self._gemm(pending[1], pending[2], chain)
-            _lib.check(_lib.lib().dlm_rowpar_bf16(C.byref(gemm), C.byref(comm), stream), f"rowpar {site}")
+            code = lib.dlm_rowpar_bf16(self._gemm(pending[1], pending[2], chain), comm, stream)
         elif fusable:  # the experts' down-projection + combine (+ shared) in front of the same reduction
-            from ..quantization import nvfp4
-
-            down = dict(pending[1])
-            shared = down.pop("shared", None)
-            m = nvfp4.descriptor(shared=shared, **down)
-            _lib.check(_lib.lib().dlm_rowpar_nvfp4_moe(C.byref(m), C.byref(comm), stream), f"experts {site}")
+            code = lib.dlm_rowpar_nvfp4_moe(pending[1].m, comm, stream)
         else:
             if pending is not None:
                 self._run_alone(pending)
-            _lib.check(_lib.lib().dlm_reduce_bf16(partial.data_ptr(), C.byref(comm), stream), f"reduce {site}")
+            code = lib.dlm_reduce_bf16(address, comm, stream)
+        if code:
+            _lib.check(code, f"{'reduce' if not fusable else 'rowpar' if pending[0] == 'linear' else 'experts'} {site}")
         self._last[chain] = out
         return out
 
@@ -362,7 +385,7 @@ class Group:
         wherever the host synchronises anyway (end of a block, end of a request)."""
         st = DlmStatus()
         stream = torch.cuda.current_stream(self.device).cuda_stream
-        _lib.check(_lib.lib().dlm_status_read(self.status.data_ptr(), C.byref(st), stream), "status")
+        _lib.check(_lib.lib().dlm_status_read(self.status.data_ptr(), st, stream), "status")
         if st.code:
             self._failed = True
             where = f"rank slot {st.slot}, phase {st.phase}, invocation {st.epoch}"
@@ -399,18 +422,19 @@ class Group:
         if self._failed:
             raise RuntimeError("this group reported a device time-out; build a new Group")
         out = self.symmetric(key, (self.world, *x.shape), x.dtype)
-        if key not in self._gather:
+        template = self._gather.get(key)
+        if template is None:
             slots = self.symmetric(key + ".slots", (3, self.world, nbytes // 2), armed=True)
             epochs = torch.zeros(_lib.EPOCH_SLOTS, device=self.device, dtype=torch.int32)
-            self._gather[key] = list(self._handles[key + ".slots"].buffer_ptrs), epochs, self.multicast(slots)
-        ptrs, epochs, recv_mc = self._gather[key]
-        c = DlmComm()
-        c.rank, c.world = self.rank, self.world
-        for s in range(self.world):
-            c.recv[s] = ptrs[s]
-        c.recv_mc = recv_mc or None
-        c.out, c.epochs, c.status = out.data_ptr(), epochs.data_ptr(), self.status.data_ptr()
-        c.timeout_ns, c.pdl, c.max_ctas = TIMEOUT_NS, int(PDL), self.max_ctas
-        stream = torch.cuda.current_stream(self.device).cuda_stream
-        _lib.check(_lib.lib().dlm_all_gather(x.data_ptr(), nbytes, C.byref(c), stream), f"all_gather {key}")
+            template = DlmComm()
+            template.rank, template.world = self.rank, self.world
+            for s, address in enumerate(self._handles[key + ".slots"].buffer_ptrs):
+                template.recv[s] = address
+            template.recv_mc = self.multicast(slots) or None
+            template.out, template.epochs, template.status = out.data_ptr(), epochs.data_ptr(), self.status.data_ptr()
+            template.keep = epochs
+            self._gather[key] = template
+        c = DlmComm.from_buffer_copy(template)
+        c.timeout_ns, c.pdl, c.max_ctas = TIMEOUT_NS, PDL, self.max_ctas
+        _lib.check(_lib.lib().dlm_all_gather(x.data_ptr(), nbytes, c, _lib.stream(self.status)), f"all_gather {key}")
         return out

@@ -10,8 +10,6 @@ FP8 activations are outside this path (the reference forces the fused reduction 
 dlmrt/models/sdar/model.py:62-64), so `fp8=True` is rejected.
 """
 
-import ctypes as C
-
 import torch
 
 from .. import _lib
@@ -58,31 +56,45 @@ class Linear:
         # Tiling of this layer's GEMM (tiles along the tokens, K splits): 0 = chosen by the library for each call.
         self.token_tiles, self.splits = token_tiles, splits
         self._workspace = None
+        self._plans = {}  # rows -> (a DlmGemm with everything filled in that no call changes, workspace bytes)
         _lib.lib()
 
     def input(self, rows, device):
         """Activation buffers this layer consumes: BF16 needs none (linear.py:34-39)."""
         return None, None
 
+    def plan(self, m):
+        """(template, workspace bytes) of this layer's GEMM over m rows. A call copies the template and sets what it
+        brings itself, so concurrent callers share nothing; filling all fields and asking the library for the size took
+        2.5 us of every call."""
+        plan = self._plans.get(m)
+        if plan is None:
+            g = DlmGemm()
+            g.m, g.n, g.k = m, self.n, self.k
+            plan = self._plans[m] = g, _lib.lib().dlm_workspace_bytes(m, self.n, self.k)
+        return plan
+
     def gemm(self, x, out, pdl=True):
         """Run the GEMM now: out[m, n] = x[m, k] @ W[n, k]^T."""
         m, k = x.shape
-        if k != self.k or tuple(out.shape) != (m, self.n) or out.dtype != torch.bfloat16 or x.dtype != torch.bfloat16:
+        if k != self.k or out.shape != (m, self.n) or out.dtype != torch.bfloat16 or x.dtype != torch.bfloat16:
             raise ValueError(f"Linear [{self.n}, {self.k}]: x {tuple(x.shape)} {x.dtype}, out {tuple(out.shape)}")
-        if x.stride(1) != 1 or out.stride(1) != 1:
+        (ldx, x_step), (ldo, out_step) = x.stride(), out.stride()
+        if x_step != 1 or out_step != 1:
             raise ValueError("x and out must have a contiguous last dimension")
-        nbytes = _lib.lib().dlm_workspace_bytes(m, self.n, k)
-        if self._workspace is None or self._workspace.numel() < nbytes:
+        template, nbytes = self.plan(m)
+        workspace = self._workspace
+        if workspace is None or workspace.numel() < nbytes:
             with torch.inference_mode(False):
-                self._workspace = torch.zeros(nbytes, device=x.device, dtype=torch.uint8)
-        g = DlmGemm()
+                workspace = self._workspace = torch.zeros(nbytes, device=x.device, dtype=torch.uint8)
+        g = DlmGemm.from_buffer_copy(template)
         self.describe(g)
-        g.x, g.m, g.n, g.k, g.ldx = x.data_ptr(), m, self.n, k, x.stride(0)
-        g.workspace, g.workspace_bytes = self._workspace.data_ptr(), self._workspace.numel()
+        g.x, g.ldx = x.data_ptr(), ldx
+        g.workspace, g.workspace_bytes = workspace.data_ptr(), workspace.numel()
         g.splits, g.token_tiles = self.splits, self.token_tiles
-        stream = torch.cuda.current_stream(x.device).cuda_stream
-        _lib.check(_lib.lib().dlm_gemm_bf16(C.byref(g), out.data_ptr(), out.stride(0), int(pdl), stream),
-                   f"gemm [{m}, {self.n}, {k}]")
+        code = _lib.lib().dlm_gemm_bf16(g, out.data_ptr(), ldo, pdl, _lib.stream(x))
+        if code:
+            _lib.check(code, f"gemm [{m}, {self.n}, {k}]")
         return out
 
     def describe(self, g):

@@ -13,7 +13,7 @@ alone, for callers that hold GEMM2's input already quantised in the expert-major
 Nothing numeric runs in Python here: tensors are only laid out and handed to libdlmrt_b200.so.
 """
 
-import ctypes as C
+from operator import is_
 
 import torch
 
@@ -160,18 +160,32 @@ def moe_down(act_codes, act_scales, amap, counts, experts, ids, weights, buffers
     reference (`rmsnorm(h, weight, delta=reduced)`, dlmrt/ops/triton/core.py:29-56) folded into the same launch.
     `replicated`: every rank holds and updates the whole residual stream (LLaDA2), see `Group.reduce_norm`."""
     m = descriptor(act_codes, act_scales, amap, counts, experts, ids, weights, buffers, num_experts, shared)
-    stream = torch.cuda.current_stream(act_codes.device).cuda_stream
     if group is None:
-        _lib.check(_lib.lib().dlm_moe_nvfp4(C.byref(m), out.data_ptr(), out.stride(0), 1, stream), "moe_down")
-        return out
+        return _run_down(m, out)
+    stream = _lib.stream(act_codes)
     mode = _lib.REDUCE if norm_weight is None else _lib.REDUCE_NORM_RESIDUAL if h is not None else _lib.REDUCE_NORM
     comm, reduced = group._comm(m.m, m.n, site, chain, mode, h, norm_weight, eps, scale, replicated and h is not None)
-    _lib.check(_lib.lib().dlm_rowpar_nvfp4_moe(C.byref(m), C.byref(comm), stream), f"moe_down {site}")
+    _lib.check(_lib.lib().dlm_rowpar_nvfp4_moe(m, comm, stream), f"moe_down {site}")
     group._last[chain] = reduced
     return reduced
 
 
 ACTIVATIONS = {"swiglu": 0, "geglu": 1}
+
+
+def _run_down(m, out):
+    """The down-projection + combine described by `m`, without a reduction behind it."""
+    code = _lib.lib().dlm_moe_nvfp4(m, out.data_ptr(), out.stride(0), 1, _lib.stream(out))
+    if code:
+        _lib.check(code, "moe_down")
+    return out
+
+
+class Down:
+    """A down-projection put off until the reduction of its output: the descriptor, and the tensors it points to."""
+
+    def __init__(self, m, *keep):
+        self.m, self.keep = m, keep
 
 
 class FrontBuffers:
@@ -192,6 +206,29 @@ class FrontBuffers:
         self.act_codes = torch.zeros(count * rows, intermediate // 2, **u8)
         self.act_scales = torch.zeros(count * rows, intermediate // 16, **u8)
         self.down = Buffers(rows, hidden, top_k, device)
+        self.sources = ()  # the experts' tensors that `front` and `back` were filled in from
+        self.front = self.back = None
+
+    def fill(self, experts, sources, num_experts):
+        """The descriptors of both halves with everything in them that no call changes. Filling 40 fields anew was half of
+        a small call's time on the host (27 us of three launches)."""
+        f = DlmMoeFront()
+        w13, s13, g1, a2_inv = sources[:4]
+        f.w13_codes, f.w13_scales = w13.data_ptr(), s13.data_ptr()
+        f.g1, f.a2_inv = g1.data_ptr(), a2_inv.data_ptr()
+        f.ids, f.weights, f.counts, f.amap = (t.data_ptr() for t in (self.ids, self.weights, self.counts, self.amap))
+        f.slot_codes, f.slot_scales = self.slot_codes.data_ptr(), self.slot_scales.data_ptr()
+        f.act_codes, f.act_scales = self.act_codes.data_ptr(), self.act_scales.data_ptr()
+        f.m, f.hidden, f.f, f.top_k, f.m_max = self.rows, experts["hidden"], experts["f"], self.ids.shape[1], self.rows
+        f.lo, f.e_local, f.e_total = experts["lo"], experts["w2"].shape[0], num_experts
+        f.w13_tiled = 1
+        self.back = descriptor(self.act_codes, self.act_scales, self.amap, self.counts, experts, self.ids, self.weights,
+                               self.down, num_experts)
+        self.sources, self.front = sources, f
+
+
+# The experts' tensors whose addresses the descriptors of a FrontBuffers hold.
+_SOURCES = ("w13", "s13", "g1", "a2_inv", "w2", "s2", "g2")
 
 
 def trtllm_moe(x, packed, experts, out, num_experts, lo, intermediate, quantized=None, activation="geglu", shared=None):
@@ -210,45 +247,39 @@ def trtllm_moe(x, packed, experts, out, num_experts, lo, intermediate, quantized
         rows, hidden = x.shape
         if x.dtype != torch.bfloat16 or not x.is_contiguous():
             raise ValueError("x must be a contiguous BF16 [rows, hidden] tensor")
-        device = x.device
     else:
-        xq, xs = quantized
-        rows, hidden = xq.shape[0], xq.shape[1] * 2
-        device = xq.device
-    count, top_k = experts["w2"].shape[0], packed.shape[1]
+        x, xs = quantized
+        rows, hidden = x.shape[0], x.shape[1] * 2
+    if packed.dtype != torch.int32 or not packed.is_contiguous():
+        raise ValueError("packed must be a contiguous int32 [rows, top_k] tensor")
     if experts["lo"] != lo or "w13" not in experts:
         raise ValueError("experts were laid out for another rank, or without their gate / up weights (b200_experts)")
     if experts["f"] != intermediate or experts["hidden"] != hidden:
         raise ValueError(f"experts are hidden {experts['hidden']}, intermediate {experts['f']}; the call says {hidden}, "
                          f"{intermediate}")
     cache = experts.setdefault("_buffers", {})
-    if rows not in cache:  # first call with this row count: before any graph capture, as the reference tunes
-        cache[rows] = FrontBuffers(rows, hidden, intermediate, count, num_experts, top_k, device)
-    b = cache[rows]
-    f = DlmMoeFront()
+    b = cache.get(rows)
+    if b is None:  # first call with this row count: before any graph capture, as the reference tunes
+        b = cache[rows] = FrontBuffers(rows, hidden, intermediate, experts["w2"].shape[0], num_experts, packed.shape[1],
+                                       x.device)
+    sources = tuple(experts[key] for key in _SOURCES)
+    if not b.sources or not all(map(is_, sources, b.sources)) or b.front.e_total != num_experts:
+        b.fill(experts, sources, num_experts)
+    f = DlmMoeFront.from_buffer_copy(b.front)
     if quantized is None:
         f.x, f.a1_inv = x.data_ptr(), experts["a1_inv"].data_ptr()
     else:
-        f.xq, f.xs = xq.data_ptr(), xs.data_ptr()
-    f.packed = packed.data_ptr()
-    f.w13_codes, f.w13_scales = experts["w13"].data_ptr(), experts["s13"].data_ptr()
-    f.g1, f.a2_inv = experts["g1"].data_ptr(), experts["a2_inv"].data_ptr()
-    f.ids, f.weights, f.counts, f.amap = b.ids.data_ptr(), b.weights.data_ptr(), b.counts.data_ptr(), b.amap.data_ptr()
-    f.slot_codes, f.slot_scales = b.slot_codes.data_ptr(), b.slot_scales.data_ptr()
-    f.act_codes, f.act_scales = b.act_codes.data_ptr(), b.act_scales.data_ptr()
-    f.m, f.hidden, f.f, f.top_k, f.m_max = rows, hidden, intermediate, top_k, rows
-    f.lo, f.e_local, f.e_total, f.activation = lo, count, num_experts, ACTIVATIONS[activation]
-    f.w13_tiled = 1
-    if packed.dtype != torch.int32 or not packed.is_contiguous():
-        raise ValueError("packed must be a contiguous int32 [rows, top_k] tensor")
-    stream = torch.cuda.current_stream(device).cuda_stream
-    _lib.check(_lib.lib().dlm_moe_front_nvfp4(C.byref(f), 1, stream), "trtllm_moe: front half")
-    down = dict(act_codes=b.act_codes, act_scales=b.act_scales, amap=b.amap, counts=b.counts, experts=experts, ids=b.ids,
-                weights=b.weights, buffers=b.down, num_experts=num_experts, shared=shared)
+        f.xq, f.xs = x.data_ptr(), xs.data_ptr()
+    f.packed, f.top_k, f.activation = packed.data_ptr(), packed.shape[1], ACTIVATIONS[activation]
+    code = _lib.lib().dlm_moe_front_nvfp4(f, 1, _lib.stream(x))
+    if code:
+        _lib.check(code, "trtllm_moe: front half")
+    m = DlmMoe.from_buffer_copy(b.back)
+    m.shared = shared.data_ptr() if shared is not None else None
     group = experts.get("group")
     if group is not None and group.is_partial(out):
-        return group.defer_experts(out, down)
-    return moe_down(out=out, **down)
+        return group.defer_experts(out, Down(m, b, sources, shared))
+    return _run_down(m, out)
 
 
 def route_packed(logits, per_expert_scale, packed, top_k):
@@ -257,9 +288,8 @@ def route_packed(logits, per_expert_scale, packed, top_k):
     rows, e = logits.shape
     if logits.dtype != torch.bfloat16 or per_expert_scale.dtype != torch.bfloat16 or packed.dtype != torch.int32:
         raise ValueError("route_packed takes BF16 logits and scales and an int32 output")
-    stream = torch.cuda.current_stream(logits.device).cuda_stream
     _lib.check(_lib.lib().dlm_route_packed(logits.contiguous().data_ptr(), per_expert_scale.data_ptr(), packed.data_ptr(),
-                                           rows, e, top_k, 1, stream), "route_packed")
+                                           rows, e, top_k, 1, _lib.stream(logits)), "route_packed")
     return packed
 
 
