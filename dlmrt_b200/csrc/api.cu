@@ -250,6 +250,11 @@ int dlm_reduce_bf16(const void* partial, const DlmComm* comm, dlm_stream_t strea
     fill_comm(&p.c[0], comm);
     p.partial[0] = static_cast<const __nv_bfloat16*>(partial);
     int grid = comm->max_ctas > 0 && comm->max_ctas < info.sms ? comm->max_ctas : info.sms;
+    if (comm->world == 1) {  // nothing is waited for inside the launch: one block per row, unless the caller caps the grid
+        if (comm->max_ctas == 0 && comm->stamps == nullptr) grid = comm->rows;
+        if (grid > comm->rows) grid = comm->rows;
+        return launch_reduce_single(p, grid, {static_cast<cudaStream_t>(stream), comm->pdl != 0, false});
+    }
     if (grid > DLM_EPOCH_SLOTS) grid = DLM_EPOCH_SLOTS;
     return launch_reduce(p, grid, comm->n / kVec, {static_cast<cudaStream_t>(stream), comm->pdl != 0, false});
 }

@@ -138,6 +138,7 @@ __device__ __forceinline__ void rearm(const CommDev& c, const CommCtx& x, int pa
     __nv_bfloat16* stale = c.recv[c.rank] + ((x.e + 2) % 3) * x.buf_elems;
     const int total = static_cast<int>(x.buf_elems / kVec);
     for (int i = first; i < total; i += stride) store_v4(stale + static_cast<size_t>(i) * kVec, sentinel);
+    if (c.world == 1) return;  // one rank collects nothing from OUT, so nobody looks for arrivals there
     for (int i = first; i < c.rearm_vecs; i += stride) store_v4(c.rearm + static_cast<size_t>(i) * kVec, sentinel);
 }
 

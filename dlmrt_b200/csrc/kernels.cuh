@@ -109,6 +109,7 @@ struct LaunchOpts {
 };
 
 int launch_reduce(const ReduceParams<1>& p, int grid, int threads, const LaunchOpts& o);
+int launch_reduce_single(const ReduceParams<1>& p, int grid, const LaunchOpts& o);
 int launch_reduce_loopback(const ReduceParams<kMaxWorld>& p, int grid, int nranks, int threads, const LaunchOpts& o);
 int launch_gather(const ReduceParams<1>& p, int grid, const LaunchOpts& o);
 int launch_gather_loopback(const ReduceParams<kMaxWorld>& p, int grid, int nranks, const LaunchOpts& o);

@@ -463,17 +463,16 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
     if (p.fused) {
         if (c.stamps && threadIdx.x == 0) c.stamps[block * kStampSlots + 6] = globaltimer();
         stamp(c, x, 1);
-        rearm_early(c, x);
-        if (local_rows) {
+        if (local_rows) {  // no slot is written, so none is re-armed and the invocation counters stay where they are
             const int* counter = g.counters + ((sm->gen + 1) & 1) * kMaxTiles;
             if (c.mode == kReduce) own_rows_from_splits<kReduce>(g, c, x, counter, mt, sm->scratch);
             else if (c.mode == kReduceNorm) own_rows_from_splits<kReduceNorm>(g, c, x, counter, mt, sm->scratch);
             else own_rows_from_splits<kReduceNormResidual>(g, c, x, counter, mt, sm->scratch);
-            rearm_late(c, x);
         } else {
+            rearm_early(c, x);
             own_and_collect(c, x, sm->scratch);  // re-arms late shares between its own and collect phases
+            comm_end(c, x);
         }
-        comm_end(c, x);
     }
 }
 

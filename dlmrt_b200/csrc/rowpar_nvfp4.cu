@@ -596,15 +596,14 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
     }
     if (p.fused) {
         stamp(c, x, 1);
-        rearm_early(c, x);
-        if (local_rows) {
+        if (local_rows) {  // no slot was written: nothing to re-arm, the invocation counters stay where they are
             stamp(c, x, 2);
             stamp(c, x, 3);
-            rearm_late(c, x);
         } else {
+            rearm_early(c, x);
             own_and_collect(c, x, sm->scratch);  // re-arms late shares between its own and collect phases
+            comm_end(c, x);
         }
-        comm_end(c, x);
     }
 }
 

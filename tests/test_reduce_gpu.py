@@ -363,3 +363,36 @@ def test_replicated_residual_stream(world, rows):
             assert_same_bits(bits(hs[r]), h_want, f"call {i}: residual stream of rank {r}")
             assert_norm_close(bits(outs[r]), want, f"call {i}: rank {r}")
             assert_same_bits(bits(outs[r]), bits(outs[0]), f"call {i}: rank {r} vs rank 0")
+
+
+@pytest.mark.parametrize("rows, n, max_ctas", [(1, 256, 0), (300, 256, 0), (3, 4096, 0), (5, 4352, 0), (150, 7936, 0), (2, 8192, 0),
+                                               (37, 2816, 4)])
+def test_one_rank_reduces_without_slots(rows, n, max_ctas):
+    """A world-1 group's reductions: one block per row (or a capped grid looping over rows), one or two vectors per thread
+    (n > 4096), a last warp of the second half left empty (n = 4352, 7936); all modes, twice over the same two sites."""
+    from dlmrt_b200.distributed.parallel import Group
+
+    g = Group.local("cuda:0")
+    g.max_ctas = max_ctas
+    weight, h = randn_bf16(n, seed=1, std=0.1) + 1, randn_bf16(rows, n, seed=2)
+    for i in range(6):
+        p, mode = randn_bf16(rows, n, seed=10 + i), i % 3
+        if mode == 0:
+            p[0, :4] = torch.tensor([-0.0, float("inf"), float("nan"), 3.0e38])
+        p_bits, h_before = bits(p)[None], bits(h)[None]
+        if mode == 0:
+            out, want = g.reduce(p, site=f"{i % 2}"), red.reduce(p_bits)
+        elif mode == 1:
+            out = g.reduce_norm(p, None, weight, 1e-6, 1.5, site=f"{i % 2}")
+            want, _ = red.reduce_norm(p_bits, bits(weight), 1e-6, 1.5)
+        else:
+            out = g.reduce_norm(p, h, weight, 1e-6, site=f"{i % 2}")
+            want, h_after = red.reduce_norm(p_bits, bits(weight), 1e-6, 1.0, h_before)
+        torch.cuda.synchronize()
+        g.check()
+        if mode == 0:
+            assert_same_bits(bits(out), want, f"call {i}")
+        else:
+            assert_norm_close(bits(out), want, f"call {i} mode {mode}")
+        if mode == 2:
+            assert_same_bits(bits(h), h_after[0], f"call {i}: residual stream")
