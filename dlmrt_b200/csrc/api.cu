@@ -523,6 +523,11 @@ static int make_map_u8(CUtensorMap* map, const void* base, long long rows, int r
     return DLM_OK;
 }
 
+static void set_layout(MoeDev* d) {
+    const MoeLayout layout = moe_layout(d->f, d->m_max, d->m * d->top_k / d->e_total);
+    d->rows_cap = layout.rows_cap, d->buffers = layout.buffers, d->stages = layout.stages;
+}
+
 static int fill_moe(MoeDev* d, const DlmMoe* m) {
     std::memset(d, 0, sizeof(*d));
     int rc = DLM_OK;
@@ -539,9 +544,7 @@ static int fill_moe(MoeDev* d, const DlmMoe* m) {
     d->y = reinterpret_cast<__nv_bfloat16*>(static_cast<char*>(m->workspace) + kWorkspaceHeader);
     d->m = m->m, d->n = m->n, d->f = m->f, d->top_k = m->top_k, d->m_max = m->m_max;
     d->lo = m->lo, d->e_local = m->e_local, d->e_total = m->e_total;
-    d->rows_cap = (m->m_max + 15) / 16 * 16;  // activation rows of one work item: at most 128
-    if (d->rows_cap > 128) d->rows_cap = 128;
-    d->stages = moe_stages(d->rows_cap);
+    set_layout(d);
     return DLM_OK;
 }
 
@@ -639,9 +642,7 @@ int dlm_moe_front_nvfp4(const DlmMoeFront* a, int pdl, dlm_stream_t stream) {
     d->m = a->m, d->n = 2 * a->f, d->f = a->hidden, d->top_k = a->top_k, d->m_max = a->m_max;
     d->lo = a->lo, d->e_local = a->e_local, d->e_total = a->e_total;
     d->f_out = a->f, d->act_kind = a->activation;
-    d->rows_cap = (a->m_max + 15) / 16 * 16;
-    if (d->rows_cap > 128) d->rows_cap = 128;
-    d->stages = moe_stages(d->rows_cap);
+    set_layout(d);
     p.fused = 0;
     return launch_moe_gate_up(p, info.sms, {s, true, false});  // always a dependent launch of the kernel above
 }

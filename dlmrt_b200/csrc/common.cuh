@@ -131,6 +131,19 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long l
     return true;
 }
 
+// The same for a whole warp that acts as one: the result is a vote, so the compiler knows it is the same in every lane.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, long long deadline) {
+    return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, deadline));
+}
+
+// A value that is the same in every lane, made known to the compiler as such. Roles that issue TMA copies or tcgen05
+// instructions run as whole warps on such values, with only the issuing instruction left to one elected lane: their
+// operands then live in uniform registers. A role that runs as `if (lane == 0)` has to move every operand there for
+// every instruction: four scale copies, four MMAs and a commit took 463 cycles of the issuing thread, 230 this way (which
+// is what the tensor pipe itself takes).
+__device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xFFFFFFFFu, v, 0); }
+__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xFFFFFFFFu, v, 0); }
+
 __device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 

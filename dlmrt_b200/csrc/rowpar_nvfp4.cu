@@ -10,15 +10,23 @@
 // point replaces dlmrt/quantization/nvfp4.py:280-306 (`trtllm_moe`) plus the add and reduce of
 // dlmrt/models/llada2/model.py:354-362,437-438.
 //
-// Work item = (active local expert, 128 output features): W2's [128 x F] slab sits on the MMA's M axis, the expert's
-// rows (tokens routed to it, padded to 16) on its N axis. Persistent CTAs take items round-robin:
-//   warp 0   TMA: per 256-element k-block the 16 KB code slab of W2 (one bulk copy of a pre-tiled slab, or one box)
-//   warp 12  TMA: the expert's activation rows of the k-block (boxes of 8 rows)
-//   warp 3   scale loader: W2's pre-interleaved 128 x 4 scale atoms and the activation rows' linear E4M3 scales,
-//            rewritten into the same atom layout, into the stage
-//   warp 1   per k-block: tcgen05.cp the scale atoms into tensor memory, then up to four
+// Work item = (entry, 128 output features), entry = (active local expert, block of at most `rows_cap` of its rows). W2's
+// [128 x F] slab sits on the MMA's M axis, the entry's rows (padded to 16) on its N axis. Every CTA takes one contiguous
+// run of items, so that consecutive items mostly share their entry and the entry's rows are fetched once per run, not
+// once per item; what streams is the weights alone:
+//   warp 0   TMA: per 256-element k-block the 16 KB code slab of W2 (one bulk copy of a pre-tiled slab, or one box) and
+//            its 2 KB of pre-interleaved 128 x 4 scale atoms (one bulk copy)
+//   warp 2   TMA, once per entry: its activation rows, all of K (boxes of 8 rows x 128 bytes)
+//   warp 3   once per entry: the rows' linear E4M3 scales, rewritten into scale atoms
+//   warp 1   per entry: tcgen05.cp the rows' scale atoms into tensor memory, where they stay for all its items (as long
+//            as K leaves room); per k-block: tcgen05.cp W2's atoms, then up to four
 //            tcgen05.mma.kind::mxf4nvf4.block_scale (K = 64) into the FP32 accumulator
-//   warps 4-11  per item: tcgen05.ld, times g2, BF16, scatter rows to Y[pair] through the expert's slot map
+//   warps 4-11  two groups of four, one accumulator buffer each, alternate items: tcgen05.ld, times g2, BF16, scatter
+//            rows to Y[pair] through the expert's slot map
+// The kernel is bound by the HBM weight stream if nothing else holds it up, and what held it up was the chain behind each
+// k-block: one thread issuing eight scale copies, four MMAs and a commit (the commit alone waits ~340 ns behind eight
+// copies), and small copies of activation rows and scales repeated for every item. Rows kept per entry halve the scale
+// copies and leave two bulk copies per k-block.
 // When all CTAs are through their items (arrival counter), rows of the output are combined from Y in FP32 and pushed
 // into the owner ranks' receive slots, and the reduction phases of comm.cuh follow.
 //
@@ -35,41 +43,76 @@ namespace dlm {
 
 namespace {
 
-constexpr int kMoeThreads = kFusedThreads + 32;  // the dense kernel's twelve warps and a second producer
+constexpr int kMoeThreads = kFusedThreads;
 constexpr int kCodeTileW = 128 * 128;  // 128 rows x 128 bytes (256 FP4) of W2 codes
 constexpr int kBoxRows = 8;            // activation rows per TMA box (one 1 KB swizzle atom)
 constexpr int kAtom = 512;             // one 128-row x 4-scale atom
 constexpr int kStepsPerBlock = 4;      // K = 64 instructions per 256-element k-block
-constexpr int kItemRows = 128;         // rows of one work item: the MMA's N; experts with more rows take several items
-constexpr int kTmemAcc = 0, kTmemSfa = 256, kTmemSfb = 384, kTmemCols = 512;  // two 128-column accumulators, then scales
-// Scale columns rotate over four sets (two per issuer: (2 * who + set) below), so copying a k-block's scales in does
-// not have to wait for the previous k-block's MMAs to finish reading theirs.
+constexpr int kStageBytes = kCodeTileW + kStepsPerBlock * kAtom;  // 18 KB: a k-block's codes and scale atoms
+constexpr int kMaxRowsCap = 128;       // rows of one entry: the MMA's N
+// Tensor memory: two 128-column accumulators, two rotating sets of W2 scale columns (a k-block's copies need not wait for
+// the previous k-block's MMAs to finish reading theirs), and the entry's row scales: four columns per K = 64 step for as
+// many steps as fit (kSfbSteps), else two rotating sets like W2's.
+constexpr int kTmemAcc = 0, kTmemSfa = 256, kTmemSfb = 288, kTmemCols = 512;
+constexpr int kSfbSteps = (kTmemCols - kTmemSfb) / 4;
 constexpr int kMaxLocalExperts = 256;
-constexpr int kMaxEntries = 2 * kMaxLocalExperts;  // (expert, row block) pairs: m_max <= 256 gives at most two blocks
+constexpr int kMaxEntries = 2 * kMaxLocalExperts;  // one per active expert + one per 16 rows of 4096 pairs at most
+constexpr int kMoeStages = 12;
+constexpr int kMoeSmemBudget = 222 * 1024;
 
 struct MoeSmem {
-    uint64_t full[kMaxStages];
-    uint64_t empty[kMaxStages];
+    uint64_t full[kMoeStages];
+    uint64_t empty[kMoeStages];
+    uint64_t a_full[2];
+    uint64_t a_empty[2];
     uint64_t acc_full[2];
     uint64_t acc_empty[2];
     uint32_t tmem_base;
     int n_active, epoch, gen, failed;
-    int seen[2];  // k-blocks (counted over this CTA's items) each issuer has seen arrive
     int warp_count[8];
     float scratch[64];
     short active[kMaxEntries];  // expert | row block << 8
     short rows[kMaxEntries];    // rows of that block
 };
 
-}  // namespace
-
-int moe_stage_bytes(int rows_cap) {  // rows_cap: rows of one item's activation tile (a multiple of 32, <= 128)
-    return kCodeTileW + rows_cap * 128 + 2 * kStepsPerBlock * kAtom;
+// Shared memory of one entry's rows: codes [k-blocks][rows_cap][128 bytes], then one scale atom per K = 64 step.
+__host__ __device__ int entry_bytes(int rows_cap, int k) {
+    return (k + 255) / 256 * rows_cap * 128 + (k / 64 + 1) / 2 * (2 * kAtom);  // a multiple of 1 KB
 }
 
-int moe_stages(int rows_cap) {
-    int s = kSmemBudget / moe_stage_bytes(rows_cap);
-    return s > kMaxStages ? kMaxStages : s;
+}  // namespace
+
+// Picks rows_cap, the number of row buffers and the ring's stages for experts of `k` inputs and at most `m_max` rows, of
+// which an expert gets `mean_rows` on average. Two buffers hide the fetch of the next entry's rows; the ring wants six
+// stages (108 KB in flight per SM cover HBM's latency at full rate), four at least. More rows per entry mean fewer
+// passes over an expert's weights (the later ones come out of L2), so the largest cap that leaves the ring its stages is
+// taken; where experts have many more rows than that on average, one larger buffer beats two small ones.
+MoeLayout moe_layout(int k, int m_max, int mean_rows) {
+    int most = (m_max + 15) / 16 * 16;
+    if (most > kMaxRowsCap) most = kMaxRowsCap;
+    auto stages_of = [&](int cap, int buffers) { return (kMoeSmemBudget - buffers * entry_bytes(cap, k)) / kStageBytes; };
+    MoeLayout best{16, 1, 1};
+    for (int want = 6; want >= 4; --want) {
+        for (int cap = most; cap >= 16; cap -= 16) {
+            if (stages_of(cap, 2) < want) continue;
+            best = {cap, 2, stages_of(cap, 2)};
+            break;
+        }
+        if (best.buffers == 2 && (best.rows_cap >= 32 || best.rows_cap == most)) break;
+    }
+    if (best.buffers == 1 || mean_rows > best.rows_cap) {
+        for (int cap = most; cap > best.rows_cap || (best.buffers == 1 && cap >= 16); cap -= 16) {
+            if (stages_of(cap, 1) < (cap == 16 ? 1 : 4)) continue;
+            best = {cap, 1, stages_of(cap, 1)};
+            break;
+        }
+    }
+    if (best.stages > kMoeStages) best.stages = kMoeStages;
+    return best;
+}
+
+static int moe_smem_bytes(const MoeDev& d) {
+    return d.stages * kStageBytes + d.buffers * entry_bytes(d.rows_cap, d.f) + static_cast<int>(sizeof(MoeSmem)) + 1024;
 }
 
 // A token's expert list for the combine step, eight entries at a time: local expert index (or -1) and routing weight.
@@ -185,39 +228,97 @@ __device__ __forceinline__ float gated_activation(float gate, float up, int kind
     return 0.5f * gate * (1.f + tanhf(inner)) * up;                  // GeGLU with the tanh GELU
 }
 
+// GEMM1's epilogue for 16 token rows x 32 tile rows (one warp): activation and NVFP4 re-quantisation. Tile row 2i holds
+// gate feature i, row 2i + 1 its up feature, so lanes l and l ^ 1 hold a feature's two halves, each for all 16 rows
+// (`r`). They swap half of them: the even lane then has both halves of rows 0-7, the odd lane of rows 8-15, and each
+// activation is computed once. The warp's 16 features are one scale block of each row, so a row's block maximum runs over
+// the 16 lanes of one parity; the maxima of eight rows are reduced together, every step halving the rows a lane still
+// carries, after which each lane holds the maximum of one row and computes that row's scale alone. One row at a time,
+// as one chain of shuffles and conversions with everything computed in two lanes, a row took 340 ns and an expert
+// with 32 rows 11 us per tile, longer than its weights take to stream.
+__device__ __forceinline__ void requantise_chunk(const MoeDev& g, const uint32_t (&r)[16], float g1, float a2i, int lane,
+                                                 int rows, int slot, int ft, int quarter) {
+    const bool odd = lane & 1;
+    float act[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const float lower = __uint_as_float(r[j]) * g1, upper = __uint_as_float(r[j + 8]) * g1;
+        const float other = __shfl_xor_sync(0xffffffff, odd ? lower : upper, 1);
+        act[j] = gated_activation(odd ? other : lower, odd ? upper : other, g.act_kind);
+    }
+    // Lane bits 4, 3, 2 choose the row each lane ends up with: `mine` = bit 4 * 4 + bit 3 * 2 + bit 2.
+    float m4[4], m2[2], amax;
+    const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float lo = fabsf(act[j]), hi = fabsf(act[j + 4]);
+        m4[j] = fmaxf(b4 ? hi : lo, __shfl_xor_sync(0xffffffff, b4 ? lo : hi, 16));
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+        m2[j] = fmaxf(b3 ? m4[j + 2] : m4[j], __shfl_xor_sync(0xffffffff, b3 ? m4[j] : m4[j + 2], 8));
+    amax = fmaxf(b2 ? m2[1] : m2[0], __shfl_xor_sync(0xffffffff, b2 ? m2[0] : m2[1], 4));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffff, amax, 2));
+    const uint32_t sf = f32_to_e4m3(a2i * (amax * rcp_approx(6.f)));
+    const float scale = amax != 0.f ? rcp_approx(e4m3_to_f32(sf) * rcp_approx(a2i)) : 0.f;
+    const int mine = (lane & 16 ? 4 : 0) + (lane & 8 ? 2 : 0) + (lane & 4 ? 1 : 0) + (odd ? 8 : 0);
+    const int groups = g.f_out / 16, half_f = g.f_out / 2;
+    if (!(lane & 2) && mine < rows)
+        g.as_out[static_cast<size_t>(slot + mine) * groups + ft * 4 + quarter] = static_cast<uint8_t>(sf);
+    // Codes: the feature's neighbour (lane ^ 2) has the other nibble of each byte. The even feature's lane assembles the
+    // bytes of rows 0-3 of its eight, the odd feature's lane those of rows 4-7.
+    const bool second = lane & 2;
+    float y[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+        y[j] = act[j] * __shfl_sync(0xffffffff, scale, (lane & 1) | (j & 4 ? 16 : 0) | (j & 2 ? 8 : 0) | (j & 1 ? 4 : 0));
+    uint8_t* codes = g.aq_out + ft * 32 + quarter * 8 + (lane >> 2);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float other = __shfl_xor_sync(0xffffffff, second ? y[j] : y[j + 4], 2);
+        const uint32_t byte = second ? e2m1x2(other, y[j + 4]) : e2m1x2(y[j], other);
+        const int row = (odd ? 8 : 0) + (second ? 4 : 0) + j;
+        if (row < rows) codes[static_cast<size_t>(slot + row) * half_f] = static_cast<uint8_t>(byte);
+    }
+}
+
 template <int NR, bool GATE_UP>
 __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_constant__ MoeParams<NR> p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const int slot = NR == 1 ? 0 : static_cast<int>(blockIdx.y);
     const MoeDev& g = p.g[slot];
     const CommDev& c = p.c[slot];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
     const int block = static_cast<int>(blockIdx.x), blocks = static_cast<int>(gridDim.x);
     if (c.stamps && threadIdx.x == 0) c.stamps[block * kStampSlots + 7] = globaltimer();
 
-    const int stage_bytes = kCodeTileW + g.rows_cap * 128 + 2 * kStepsPerBlock * kAtom;
-    const int off_a = kCodeTileW, off_sfa = off_a + g.rows_cap * 128, off_sfb = off_sfa + kStepsPerBlock * kAtom;
     const int feature_tiles = g.n / kBlockF;
     const int steps = g.f / 64;                  // K = 64 instructions per item
     const int nkb = (steps + kStepsPerBlock - 1) / kStepsPerBlock;
     const int scale_row = g.f / 16;              // bytes of scales per activation row
+    const int row_tile = g.rows_cap * 128;       // bytes of one k-block of an entry's rows
+    const int rows_bytes = entry_bytes(g.rows_cap, g.f);
 
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    MoeSmem* sm = reinterpret_cast<MoeSmem*>(tiles + g.stages * stage_bytes);
+    // The ring's codes, then its scale atoms, then the entries' rows: everything the MMAs read swizzled is 1 KB aligned.
+    uint8_t* ring_scales = tiles + g.stages * kCodeTileW;
+    uint8_t* entry_rows = tiles + g.stages * kStageBytes;
+    MoeSmem* sm = reinterpret_cast<MoeSmem*>(entry_rows + g.buffers * rows_bytes);
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < g.stages; ++i) {
-            mbar_init(&sm->full[i], 33);  // the TMA producer's expect_tx arrival and the scale loader's 32 lanes
+            mbar_init(&sm->full[i], 1);
             mbar_init(&sm->empty[i], 1);
         }
         for (int i = 0; i < 2; ++i) {
+            mbar_init(&sm->a_full[i], 33);  // the TMA producer's expect_tx arrival and the scale loader's 32 lanes
+            mbar_init(&sm->a_empty[i], 1);
             mbar_init(&sm->acc_full[i], 1);
-            mbar_init(&sm->acc_empty[i], 8);  // one arrival per epilogue warp
+            mbar_init(&sm->acc_empty[i], 4);  // one arrival per epilogue warp of the buffer's group
         }
         fence_barrier_init();
-        tma_prefetch_descriptor(&g.tm_w);
+        if (!g.w_tiles) tma_prefetch_descriptor(&g.tm_w);
         tma_prefetch_descriptor(&g.tm_a);
-        sm->seen[0] = sm->seen[1] = 0;
     }
     if (warp == 2) tmem_alloc(&sm->tmem_base, kTmemCols);
     // The next kernel of the stream may be set up from now on (its blocks move in as this kernel's blocks leave).
@@ -225,7 +326,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
     // Routing (counts, slots, activations) comes from the previous kernels of the stream: nothing of it may be read
     // before they are complete.
     pdl_wait();
-    // Compact list of (expert, block of 128 rows) pairs that have rows, in expert order.
+    // Compact list of (expert, block of rows_cap rows) entries that have rows, in expert order.
     {
         const int e = threadIdx.x;
         const int total_rows = e < g.e_local ? min(g.counts[g.lo + e], g.m_max) : 0;
@@ -235,7 +336,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
             if (threadIdx.x == 353) early = g.gen[block];
             if (threadIdx.x == 354 && p.fused) early = comm_failed(c);
         }
-        const int nb = (total_rows + kItemRows - 1) / kItemRows;
+        const int nb = (total_rows + g.rows_cap - 1) / g.rows_cap;
         int incl = nb;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -249,14 +350,14 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
         if (warp < 8) {
             int base = 0;
             for (int wv = 0; wv < warp; ++wv) base += sm->warp_count[wv];
-            for (int j = 0; j < nb; ++j) {
+            for (int j = 0; j < nb && base + incl - nb + j < kMaxEntries; ++j) {
                 sm->active[base + incl - nb + j] = static_cast<short>(e | (j << 8));
-                sm->rows[base + incl - nb + j] = static_cast<short>(min(total_rows - j * kItemRows, kItemRows));
+                sm->rows[base + incl - nb + j] = static_cast<short>(min(total_rows - j * g.rows_cap, g.rows_cap));
             }
             if (threadIdx.x == 0) {
                 int total = 0;
                 for (int wv = 0; wv < 8; ++wv) total += sm->warp_count[wv];
-                sm->n_active = total;
+                sm->n_active = min(total, kMaxEntries);
             }
         }
         if (threadIdx.x == 352) sm->epoch = early;
@@ -265,273 +366,219 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
         __syncthreads();
     }
     if (c.stamps && threadIdx.x == 0) c.stamps[block * kStampSlots + 0] = globaltimer();
-    const uint32_t tmem = sm->tmem_base;
-    const int n_items = sm->n_active * feature_tiles;
+    const uint32_t tmem = uniform(sm->tmem_base);
+    const int n_items = uniform(sm->n_active) * feature_tiles;
     const long long deadline = globaltimer() + (c.timeout_ns > 0 ? c.timeout_ns : kDefaultTimeoutNs);
 
-    // An item: entry (expert e, row block rb) x feature tile ft; `cnt` rows of the expert starting at row0.
-    struct Item {
-        int e, ft, row0, cnt;
-    };
-    auto item_of = [&](int i) {
-        const int entry = sm->active[i / feature_tiles];
-        Item t;
-        t.e = entry & 0xFF, t.ft = i % feature_tiles, t.row0 = (entry >> 8) * kItemRows;
-        t.cnt = sm->rows[i / feature_tiles];
-        return t;
-    };
-
-    if (warp == 0) {
-        if (lane == 0) {
-            int st = 0;
-            uint32_t phase = 1;  // waiting for parity 1 on a fresh barrier returns at once: the first lap is free
-            for (int i = block; i < n_items; i += blocks) {
-                const Item t = item_of(i);
-                const int boxes = (t.cnt + kBoxRows - 1) / kBoxRows;
-                for (int kb = 0; kb < nkb; ++kb) {
-                    if (!mbar_wait(&sm->empty[st], phase, deadline)) {
-                        report(c.status, kErrTimeout, st, kPhasePipeline, 0);
-                        i = n_items;
-                        break;
-                    }
-                    uint8_t* stage = tiles + st * stage_bytes;
-                    mbar_expect_tx(&sm->full[st], static_cast<uint32_t>(kCodeTileW + boxes * kBoxRows * 128));
-                    if (g.w_tiles)  // one contiguous 16 KB run of HBM, already in the swizzled shared-memory order
-                        bulk_load(stage, g.w_tiles + (static_cast<size_t>(t.e * feature_tiles + t.ft) * nkb + kb) * kCodeTileW,
-                                  kCodeTileW, &sm->full[st], kEvictFirst);
-                    else
-                        tma_load_2d(stage, &g.tm_w, &sm->full[st], kb * 128, t.e * g.n + t.ft * kBlockF, kEvictFirst);
-                    if (++st == g.stages) st = 0, phase ^= 1;
-                }
-            }
+    // This CTA's run of items, and its position in it: entry and feature tile advance together.
+    struct Cursor {
+        int entry, ft;
+        __device__ void next(int feature_tiles) {
+            if (++ft == feature_tiles) ft = 0, ++entry;
         }
-        __syncwarp();  // lanes 1-31 must not run ahead to the block-wide barrier while lane 0 is still issuing
-    } else if (warp == 12) {
-        // Second producer: the expert's activation rows (boxes of 8 rows), so that the thread that requests the weight
-        // slabs has one copy per k-block to issue (config 5, several boxes per k-block: 47.9 instead of 49.5 us per
-        // layer; config 4: no change). It only adds bytes to a phase the weight producer announces.
-        if (lane == 0) {
-            int st = 0;
-            uint32_t phase = 1;
-            for (int i = block; i < n_items; i += blocks) {
-                const Item t = item_of(i);
-                const int boxes = (t.cnt + kBoxRows - 1) / kBoxRows;
-                for (int kb = 0; kb < nkb; ++kb) {
-                    if (!mbar_wait(&sm->empty[st], phase, deadline)) {
-                        report(c.status, kErrTimeout, st, kPhasePipeline, 0);
-                        i = n_items;
-                        break;
-                    }
-                    uint8_t* stage = tiles + st * stage_bytes;
-                    for (int b = 0; b < boxes; ++b)
-                        tma_load_2d(stage + off_a + b * kBoxRows * 128, &g.tm_a, &sm->full[st], kb * 128,
-                                    t.e * g.m_max + t.row0 + b * kBoxRows, kEvictLast);
-                    if (++st == g.stages) st = 0, phase ^= 1;
+    };
+    const int i0 = static_cast<int>(static_cast<long long>(block) * n_items / blocks);
+    const int i1 = static_cast<int>(static_cast<long long>(block + 1) * n_items / blocks);
+    const int first_entry = i0 / feature_tiles;
+    const int last_entry = i1 > i0 ? (i1 - 1) / feature_tiles : first_entry - 1;
+    const Cursor start{first_entry, i0 - first_entry * feature_tiles};
+
+    // Warps 0 to 2 run as whole warps on uniform values, one elected lane issuing (see uniform()).
+    if (warp == 0) {
+        const bool leader = elect_one();
+        int st = 0;
+        uint32_t phase = 1;  // waiting for parity 1 on a fresh barrier returns at once: the first lap is free
+        Cursor at = start;
+        for (int i = i0; i < i1; ++i, at.next(feature_tiles)) {
+            const int e = uniform(sm->active[at.entry] & 0xFF);
+            const size_t tile = static_cast<size_t>(e) * feature_tiles + at.ft;
+            const uint8_t* codes = g.w_tiles + tile * nkb * kCodeTileW;
+            const uint8_t* scales = g.w_scales + tile * steps * kAtom;
+            for (int kb = 0; kb < nkb; ++kb) {
+                if (!mbar_wait_warp(&sm->empty[st], phase, deadline)) {
+                    if (leader) report(c.status, kErrTimeout, st, kPhasePipeline, 0);
+                    i = i1;
+                    break;
                 }
+                const uint32_t scale_bytes = static_cast<uint32_t>(min(kStepsPerBlock, steps - kb * kStepsPerBlock)) * kAtom;
+                if (leader) {
+                    mbar_expect_tx(&sm->full[st], kCodeTileW + scale_bytes);
+                    if (g.w_tiles)  // one contiguous 16 KB run of HBM, already in the swizzled shared-memory order
+                        bulk_load(tiles + st * kCodeTileW, codes + kb * kCodeTileW, kCodeTileW, &sm->full[st], kEvictFirst);
+                    else
+                        tma_load_2d(tiles + st * kCodeTileW, &g.tm_w, &sm->full[st], kb * 128, e * g.n + at.ft * kBlockF,
+                                    kEvictFirst);
+                    bulk_load(ring_scales + st * kStepsPerBlock * kAtom, scales + kb * kStepsPerBlock * kAtom, scale_bytes,
+                              &sm->full[st], kEvictFirst);
+                }
+                if (++st == g.stages) st = 0, phase ^= 1;
             }
         }
         __syncwarp();
-    } else if (warp == 3) {
-        // Scale loader: asynchronous copies straight into the atoms, so it never waits for data and runs as far ahead
-        // as the ring allows. Atom byte (r % 32) * 16 + (r / 32) * 4 + j holds scale j of row r (< 128).
-        const int last_slot = g.e_local * g.m_max - 1;
-        int st = 0;
+    } else if (warp == 2 || warp == 3) {
+        // The entries' rows: codes by TMA (warp 2, one thread), scales by asynchronous copies straight into the atoms
+        // (warp 3): atom byte (r % 32) * 16 + (r / 32) * 4 + j of step s holds scale 4 s + j of row r (< 128). A buffer is
+        // refilled once the MMAs of the entry it held have completed.
+        const bool leader = elect_one();
+        int buf = 0;
         uint32_t phase = 1;
-        for (int i = block; i < n_items; i += blocks) {
-            const Item t = item_of(i);
-            const int rows = (t.cnt + 15) & ~15;  // the MMA reads scales of all its N rows
-            bool alive = true;
+        for (int entry = first_entry; entry <= last_entry; ++entry) {
+            if (!mbar_wait_warp(&sm->a_empty[buf], phase, deadline)) {
+                if (leader) report(c.status, kErrTimeout, buf, kPhasePipeline, 5);
+                break;
+            }
+            const int what = uniform(static_cast<int>(sm->active[entry])), cnt = uniform(static_cast<int>(sm->rows[entry]));
+            const int row0 = (what & 0xFF) * g.m_max + (what >> 8) * g.rows_cap;  // first slot of the entry
+            uint8_t* rows = entry_rows + buf * rows_bytes;
+            if (warp == 2) {
+                const int boxes = (cnt + kBoxRows - 1) / kBoxRows;
+                if (leader) {
+                    mbar_expect_tx(&sm->a_full[buf], static_cast<uint32_t>(nkb * boxes * kBoxRows * 128));
+                    for (int kb = 0; kb < nkb; ++kb)
+                        for (int b = 0; b < boxes; ++b)
+                            tma_load_2d(rows + kb * row_tile + b * kBoxRows * 128, &g.tm_a, &sm->a_full[buf], kb * 128,
+                                        row0 + b * kBoxRows, kEvictLast);
+                }
+            } else {
+                uint8_t* atoms = rows + nkb * row_tile;
+                for (int r = 0; r < cnt; ++r) {
+                    const uint8_t* src = g.a_scales + static_cast<size_t>(row0 + r) * scale_row;
+                    uint8_t* dst = atoms + (r % 32) * 16 + (r / 32) * 4;
+                    for (int s2 = lane; s2 < steps; s2 += 32) cp_async_4(dst + s2 * kAtom, src + s2 * 4);
+                }
+                cp_async_arrive(&sm->a_full[buf]);
+            }
+            if (++buf == g.buffers) buf = 0, phase ^= 1;
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        // One lane feeds the tensor pipe, so everything it issues executes in that order: scale copies into columns
+        // that earlier MMAs read need no wait.
+        const bool leader = elect_one();
+        const uint64_t desc_hi = umma_desc_k128(tiles) & 0xFFFFFFFF00000000ull;     // swizzled operand tiles
+        const uint64_t sf_hi = utccp_desc(tiles) & 0xFFFFFFFF00000000ull;           // scale atoms
+        auto operand = [&](uint32_t address) { return desc_hi | ((address & 0x3FFFF) >> 4); };
+        auto atom = [&](uint32_t address) { return sf_hi | ((address & 0x3FFFF) >> 4); };
+        const uint32_t ring = smem_u32(tiles), scales = smem_u32(ring_scales), rows0 = smem_u32(entry_rows);
+        const bool resident = steps <= kSfbSteps;  // the entry's row scales stay in tensor memory
+        int st = 0, set = 0, buf = -1;
+        uint32_t phase = 0, a_phase = 1;
+        uint32_t rows = 0, idesc = 0;
+        bool alive = true;
+        Cursor at = start;
+        for (int i = i0; i < i1 && alive; ++i, at.next(feature_tiles)) {
+            const int item = i - i0, acc_buf = item & 1;
+            if (item == 0 || at.ft == 0) {  // a new entry
+                if (leader && buf >= 0) umma_commit(&sm->a_empty[buf]);
+                if (++buf == g.buffers) buf = 0;
+                if (buf == 0) a_phase ^= 1;
+                if (!mbar_wait_warp(&sm->a_full[buf], a_phase, deadline)) {
+                    if (leader) report(c.status, kErrTimeout, buf, kPhasePipeline, 6);
+                    break;
+                }
+                fence_proxy_async();  // the scale atoms were written through the generic proxy
+                tcgen05_fence_after();
+                rows = rows0 + buf * rows_bytes;
+                idesc = umma_idesc_nvfp4(kBlockF, (uniform(static_cast<int>(sm->rows[at.entry])) + 15) & ~15);
+                if (resident && leader)
+                    for (int s2 = 0; s2 < steps; ++s2)
+                        utccp_128x4(tmem + kTmemSfb + 4 * s2, atom(rows + nkb * row_tile + s2 * kAtom));
+            }
+            // The accumulator buffer must have been read out by the epilogue of two items ago.
+            if (item >= 2 && !mbar_wait_warp(&sm->acc_empty[acc_buf], ((item >> 1) - 1) & 1, deadline)) {
+                if (leader) report(c.status, kErrTimeout, 0, kPhasePipeline, 4);
+                break;
+            }
+            tcgen05_fence_after();
+            const uint32_t acc = tmem + kTmemAcc + acc_buf * kMaxRowsCap;
             for (int kb = 0; kb < nkb; ++kb) {
-                if (!mbar_wait(&sm->empty[st], phase, deadline)) {
+                if (!mbar_wait_warp(&sm->full[st], phase, deadline)) {
+                    if (leader) report(c.status, kErrTimeout, st, kPhasePipeline, 1);
                     alive = false;
                     break;
                 }
-                uint8_t* stage = tiles + st * stage_bytes;
+                tcgen05_fence_after();
+                const uint64_t dw = operand(ring + st * kCodeTileW), da = operand(rows + kb * row_tile);
+                const uint64_t fa = atom(scales + st * kStepsPerBlock * kAtom);
+                const uint32_t sfa = tmem + kTmemSfa + set * 4 * kStepsPerBlock;
+                const uint32_t sfb = tmem + kTmemSfb + 4 * kStepsPerBlock * (resident ? kb : set);
                 const int nsteps = min(kStepsPerBlock, steps - kb * kStepsPerBlock);
-                const uint8_t* wsrc =
-                    g.w_scales + (static_cast<size_t>(t.e * feature_tiles + t.ft) * steps + kb * kStepsPerBlock) * kAtom;
-                for (int v = lane; v < nsteps * (kAtom / 16); v += 32) cp_async_16(stage + off_sfa + v * 16, wsrc + v * 16);
-                for (int r = lane; r < rows; r += 32) {
-                    // Rows past the expert's count are padding: any readable scale will do for them.
-                    const int srow = min(t.e * g.m_max + t.row0 + r, last_slot);
-                    const uint8_t* src = g.a_scales + static_cast<size_t>(srow) * scale_row + kb * kStepsPerBlock * 4;
-                    uint8_t* dst = stage + off_sfb + (r % 32) * 16 + (r / 32) * 4;
-                    for (int s2 = 0; s2 < nsteps; ++s2) cp_async_4(dst + s2 * kAtom, src + s2 * 4);
-                }
-                cp_async_arrive(&sm->full[st]);
-                if (++st == g.stages) st = 0, phase ^= 1;
-            }
-            if (!alive) break;
-        }
-    } else if (warp == 1 || warp == 2) {
-        // Two threads feed the tensor pipe: warp 1 takes this CTA's even work items, warp 2 the odd ones. Each item has
-        // its own accumulator buffer anyway (item & 1), and each issuer its own two sets of scale columns, so the two
-        // instruction streams never touch the same tensor memory. One thread alone is the bottleneck of the stream:
-        // per 256-element k-block it waits on a barrier, issues eight scale copies and four MMAs and commits. Ring
-        // position, phase and scale set advance by increments (no divisions); descriptors differ by constants.
-        const int who = warp - 1;
-        if (lane == 0) {
-            const uint32_t stage0 = smem_u32(tiles);
-            const uint64_t desc_hi = umma_desc_k128(tiles) & 0xFFFFFFFF00000000ull;     // swizzled operand tiles
-            const uint64_t sf_hi = utccp_desc(tiles) & 0xFFFFFFFF00000000ull;           // scale atoms
-            int st = 0, set = 0, item = 0, seq = 0;  // seq: this k-block's number in the CTA's sequence
-            uint32_t phase = 0;
-            bool alive = true;
-            // A parity wait tells a barrier's phases apart only while the waiter is never a whole phase behind, and an
-            // issuer skips the phases of the other's items. So before it waits for k-block `seq` it makes sure that
-            // k-block `seq - stages` (the same stage's previous phase) has been seen to arrive by whoever owns it; the
-            // two publish what they have seen in shared memory. That k-block belongs to the other issuer iff the
-            // number of items between the two is odd: (stages / nkb), or one more for the first stages % nkb k-blocks
-            // of an item.
-            const int q_items = g.stages / nkb, r_blocks = g.stages % nkb;
-            volatile int* seen = sm->seen;
-            const bool guarded = (q_items & 1) || r_blocks != 0;  // otherwise a stage always belongs to the same issuer
-            for (int i = block; i < n_items && alive; i += blocks, ++item) {
-                if ((item & 1) != who) {  // the other issuer's item: only step over its k-blocks in the ring
-                    st += nkb;
-                    seq += nkb;
-                    while (st >= g.stages) st -= g.stages, phase ^= 1;
-                    continue;
-                }
-                const int cnt = sm->rows[i / feature_tiles];
-                const uint32_t idesc = umma_idesc_nvfp4(kBlockF, max(16, (cnt + 15) & ~15));
-                const uint32_t acc = tmem + kTmemAcc + who * kItemRows;
-                // The accumulator buffer must have been read out by the epilogue of two items ago.
-                if (item >= 2 && !mbar_wait(&sm->acc_empty[who], ((item >> 1) - 1) & 1, deadline)) {
-                    report(c.status, kErrTimeout, 0, kPhasePipeline, 4);
-                    break;
-                }
-                for (int kb = 0; kb < nkb; ++kb, ++seq) {
-                    if (guarded && seq >= g.stages && ((kb >= r_blocks ? q_items : q_items + 1) & 1)) {
-                        while (alive && seen[1 - who] <= seq - g.stages) alive = globaltimer() <= deadline;
+                if (leader) {
+                    if (!resident) {
+                        const uint64_t fb = atom(rows + nkb * row_tile + kb * kStepsPerBlock * kAtom);
+                        for (int s2 = 0; s2 < nsteps; ++s2) utccp_128x4(sfb + 4 * s2, fb + s2 * (kAtom >> 4));
                     }
-                    if (!alive || !mbar_wait(&sm->full[st], phase, deadline)) {
-                        report(c.status, kErrTimeout, st, kPhasePipeline, 1);
-                        alive = false;
-                        break;
-                    }
-                    if (guarded) seen[who] = seq + 1;
-                    fence_proxy_async();  // the scale atoms were written through the generic proxy
-                    tcgen05_fence_after();
-                    const uint32_t base = stage0 + st * stage_bytes;
-                    const uint64_t dw = desc_hi | ((base & 0x3FFFF) >> 4), da = desc_hi | (((base + off_a) & 0x3FFFF) >> 4);
-                    const uint64_t fa = sf_hi | (((base + off_sfa) & 0x3FFFF) >> 4), fb = sf_hi | (((base + off_sfb) & 0x3FFFF) >> 4);
-                    const uint32_t sfa = tmem + kTmemSfa + (2 * who + set) * 4 * kStepsPerBlock;
-                    const uint32_t sfb = tmem + kTmemSfb + (2 * who + set) * 4 * kStepsPerBlock;
-                    const int nsteps = min(kStepsPerBlock, steps - kb * kStepsPerBlock);
                     if (nsteps == kStepsPerBlock) {
 #pragma unroll
-                        for (int s2 = 0; s2 < kStepsPerBlock; ++s2) {
-                            utccp_128x4(sfa + 4 * s2, fa + s2 * (kAtom >> 4));
-                            utccp_128x4(sfb + 4 * s2, fb + s2 * (kAtom >> 4));
-                        }
+                        for (int s2 = 0; s2 < kStepsPerBlock; ++s2) utccp_128x4(sfa + 4 * s2, fa + s2 * (kAtom >> 4));
 #pragma unroll
                         for (int s2 = 0; s2 < kStepsPerBlock; ++s2)
                             umma_nvfp4(acc, dw + 2 * s2, da + 2 * s2, idesc, sfa + 4 * s2, sfb + 4 * s2, (kb | s2) != 0);
                     } else {
-                        for (int s2 = 0; s2 < nsteps; ++s2) {
-                            utccp_128x4(sfa + 4 * s2, fa + s2 * (kAtom >> 4));
-                            utccp_128x4(sfb + 4 * s2, fb + s2 * (kAtom >> 4));
-                        }
+                        for (int s2 = 0; s2 < nsteps; ++s2) utccp_128x4(sfa + 4 * s2, fa + s2 * (kAtom >> 4));
                         for (int s2 = 0; s2 < nsteps; ++s2)
                             umma_nvfp4(acc, dw + 2 * s2, da + 2 * s2, idesc, sfa + 4 * s2, sfb + 4 * s2, (kb | s2) != 0);
                     }
                     umma_commit(&sm->empty[st]);
-                    set ^= 1;
-                    if (++st == g.stages) st = 0, phase ^= 1;
                 }
-                if (alive) umma_commit(&sm->acc_full[who]);
+                set ^= 1;
+                if (++st == g.stages) st = 0, phase ^= 1;
             }
+            if (alive && leader) umma_commit(&sm->acc_full[acc_buf]);
         }
         __syncwarp();
-    } else if (warp >= 4 && warp < 12) {
-        // Epilogue: lane = output feature of the tile, registers = the expert's rows.
-        const int quarter = warp & 3, half = (warp - 4) >> 2;
-        int item = 0;
-        // What an item's epilogue needs from global memory: the expert's scale(s) and, for the down-projection, for each
-        // of this warp's 16-row chunks (at most four) the destination row of lane % 16's accumulator column. Fetched
-        // one item AHEAD: the epilogue warps go from item to item without a pause when the stream runs well, and a
-        // round trip to L2 per item would then set the pace of the whole CTA.
-        struct Meta {
-            float g2, a2i;
-            int dest[4];
-        };
-        auto fetch = [&](int i) {
-            Meta m{0.f, 0.f, {-1, -1, -1, -1}};
-            if (i >= n_items) return m;
-            const Item t = item_of(i);
-            m.g2 = g.g2[t.e];
-            if (GATE_UP) {
-                m.a2i = g.a2_inv[t.e];
-            } else {
-                const int* slots = g.amap + static_cast<size_t>(g.lo + t.e) * g.m_max + t.row0;
+    } else {
+        // Epilogue: lane = output feature of the tile, registers = the entry's rows. Group 0 takes the run's even items,
+        // group 1 the odd ones. What it needs from global memory (the expert's scale, the destination rows) changes with
+        // the entry only.
+        const int quarter = warp & 3, group = (warp - 4) >> 2;
+        int entry = -1, cnt = 0, slot0 = 0;
+        float g2 = 0.f, a2i = 0.f;
+        int dest[kMaxRowsCap / 32];  // destination of row 32 q + lane
+        Cursor at = start;
+        if (group == 1) at.next(feature_tiles);
+        for (int i = i0 + group; i < i1; i += 2, at.next(feature_tiles), at.next(feature_tiles)) {
+            if (at.entry != entry) {
+                entry = at.entry;
+                const int what = sm->active[entry], e = what & 0xFF, row0 = (what >> 8) * g.rows_cap;
+                cnt = sm->rows[entry];
+                g2 = g.g2[e];
+                if (GATE_UP) {
+                    a2i = g.a2_inv[e];
+                    slot0 = e * g.m_max + row0;
+                } else {
+                    const int* slots = g.amap + static_cast<size_t>(g.lo + e) * g.m_max + row0;
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int row = (half + 2 * q) * 16 + (lane & 15);
-                    m.dest[q] = row < t.cnt ? slots[row] : -1;
+                    for (int q = 0; q < kMaxRowsCap / 32; ++q) dest[q] = q * 32 + lane < cnt ? slots[q * 32 + lane] : -1;
                 }
             }
-            return m;
-        };
-        Meta next = fetch(block);
-        for (int i = block; i < n_items; i += blocks, ++item) {
-            const Item t = item_of(i);
-            const int n_mma = max(16, (t.cnt + 15) & ~15);
-            const int buf = item & 1;
-            const Meta cur = next;
-            next = fetch(i + blocks);
-            const float g2 = cur.g2, a2i = cur.a2i;
-            const int(&dest)[4] = cur.dest;
-            const bool ok = mbar_wait(&sm->acc_full[buf], (item >> 1) & 1, deadline);
-            if (!ok) report(c.status, kErrTimeout, 0, kPhasePipeline, 2);
+            if (!mbar_wait(&sm->acc_full[group], ((i - i0) >> 1) & 1, deadline)) {
+                report(c.status, kErrTimeout, 0, kPhasePipeline, 2);
+                break;
+            }
             tcgen05_fence_after();
-            const int col = t.ft * kBlockF + quarter * 32 + lane;
+            const int col = at.ft * kBlockF + quarter * 32 + lane;
+            const uint32_t acc = tmem + kTmemAcc + group * kMaxRowsCap + (static_cast<uint32_t>(quarter * 32) << 16);
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int chunk = half + 2 * q;
-                if (chunk < n_mma / 16 && ok) {
-                    uint32_t r[16];
-                    tmem_load_16(tmem + kTmemAcc + buf * kItemRows + (static_cast<uint32_t>(quarter * 32) << 16) + chunk * 16, r);
-                    tmem_load_wait();
-                    if (GATE_UP) {
-                        // Tile row 2i holds gate feature i, row 2i + 1 its up feature: neighbouring lanes. The warp's 32
-                        // lanes are one block of 16 activation features (ft * 64 + quarter * 16 ..) of 16 token rows.
-                        const size_t slot0 = static_cast<size_t>(t.e) * g.m_max + t.row0;
-                        const int half_f = g.f_out / 2, groups = g.f_out / 16;
+            for (int chunk = 0; chunk < kMaxRowsCap / 16; ++chunk) {
+                if (chunk * 16 >= cnt) break;
+                uint32_t r[16];
+                tmem_load_16(acc + chunk * 16, r);
+                tmem_load_wait();
+                if (GATE_UP) {
+                    requantise_chunk(g, r, g2, a2i, lane, cnt - chunk * 16, slot0 + chunk * 16, at.ft, quarter);
+                } else {
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            const float mine = __uint_as_float(r[j]) * g2;
-                            const float other = __shfl_xor_sync(0xffffffff, mine, 1);
-                            const float act = gated_activation(lane & 1 ? other : mine, lane & 1 ? mine : other, g.act_kind);
-                            float amax = fabsf(act);
-#pragma unroll
-                            for (int o = 2; o < 32; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffff, amax, o));
-                            const uint32_t sf = f32_to_e4m3(a2i * (amax * rcp_approx(6.f)));
-                            const float scale = amax != 0.f ? rcp_approx(e4m3_to_f32(sf) * rcp_approx(a2i)) : 0.f;
-                            const float y = act * scale;
-                            const float y_next = __shfl_down_sync(0xffffffff, y, 2);  // the next feature's value
-                            const int row = chunk * 16 + j;
-                            if (row < t.cnt) {
-                                if ((lane & 3) == 0)
-                                    g.aq_out[(slot0 + row) * half_f + t.ft * 32 + quarter * 8 + (lane >> 2)] =
-                                        static_cast<uint8_t>(e2m1x2(y, y_next));
-                                if (lane == 0) g.as_out[(slot0 + row) * groups + t.ft * 4 + quarter] = static_cast<uint8_t>(sf);
-                            }
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            const int pair = __shfl_sync(0xffffffff, dest[q], j);
-                            if (pair >= 0)
-                                g.y[static_cast<size_t>(pair) * g.n + col] = __float2bfloat16_rn(__uint_as_float(r[j]) * g2);
-                        }
+                    for (int j = 0; j < 16; ++j) {
+                        const int pair = __shfl_sync(0xffffffff, dest[chunk / 2], (chunk & 1) * 16 + j);
+                        if (pair >= 0)
+                            g.y[static_cast<size_t>(pair) * g.n + col] = __float2bfloat16_rn(__uint_as_float(r[j]) * g2);
                     }
                 }
             }
             tcgen05_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sm->acc_empty[buf]);
-            if (!ok) break;
+            if (lane == 0) mbar_arrive(&sm->acc_empty[group]);
         }
     }
     // Every Y row this CTA produced is written; announce it and wait for the rest of the grid (the combine reads rows
@@ -609,14 +656,14 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
 
 template <int NR, bool GATE_UP>
 static int launch_impl(const MoeParams<NR>& p, dim3 grid, const LaunchOpts& o) {
-    const int smem = p.g[0].stages * moe_stage_bytes(p.g[0].rows_cap) + static_cast<int>(sizeof(MoeSmem)) + 1024;
+    const int smem = moe_smem_bytes(p.g[0]);
     static bool raised[64] = {};
     cudaError_t err = cudaSuccess;
     int dev = 0;
     (void)cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !raised[dev]) {
         err = cudaFuncSetAttribute(moe_kernel<NR, GATE_UP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   kSmemBudget + static_cast<int>(sizeof(MoeSmem)) + 1024);
+                                   kMoeSmemBudget + static_cast<int>(sizeof(MoeSmem)) + 1024);
         raised[dev] = err == cudaSuccess;
     }
     if (err == cudaSuccess) {
