@@ -98,9 +98,6 @@ SIGNATURES = {
     "dlm_rowpar_nvfp4_moe_loopback": (C.c_int, [C.POINTER(DlmMoe), C.POINTER(DlmComm), C.c_int, C.c_void_p]),
     "dlm_moe_workspace_bytes": (C.c_size_t, [C.c_int, C.c_int, C.c_int]),
     "dlm_moe_front_nvfp4": (C.c_int, [C.POINTER(DlmMoeFront), C.c_int, C.c_void_p]),
-    "dlm_moe_experts_nvfp4": (C.c_int, [C.POINTER(DlmMoeFront), C.POINTER(DlmMoe), C.c_int, C.c_void_p]),
-    "dlm_moe_combine": (C.c_int, [C.POINTER(DlmMoe), C.c_void_p, C.c_int64, C.c_int, C.c_void_p]),
-    "dlm_rowpar_moe_combine": (C.c_int, [C.POINTER(DlmMoe), C.POINTER(DlmComm), C.c_void_p]),
     "dlm_route_packed": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p]),
     "dlm_abi_check_front": (C.c_int, [C.c_size_t]),
     "dlm_abi_check_moe": (C.c_int, [C.c_size_t]),

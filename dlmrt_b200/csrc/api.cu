@@ -523,53 +523,34 @@ static int make_map_u8(CUtensorMap* map, const void* base, long long rows, int r
     return DLM_OK;
 }
 
-// Shared memory of an expert launch, sized for the longer of the K that its rows have.
 static void set_layout(MoeDev* d) {
-    const int k = d->gemm[0].n > 0 && d->gemm[0].k > d->gemm[1].k ? d->gemm[0].k : d->gemm[1].k;
-    const MoeLayout layout = moe_layout(k, d->m_max, d->m * d->top_k / d->e_total);
+    const MoeLayout layout = moe_layout(d->f, d->m_max, d->m * d->top_k / d->e_total);
     d->rows_cap = layout.rows_cap, d->buffers = layout.buffers, d->stages = layout.stages;
 }
 
-static int fill_gemm_half(ExpertGemm* w, const void* codes, int tiled, const void* scales, const void* rows,
-                          const void* row_scales, const float* alpha, int e_local, int m_max, int n, int k) {
-    int rc = DLM_OK;
-    if (tiled) w->w_tiles = static_cast<const uint8_t*>(codes);
-    else rc = make_map_u8(&w->tm_w, codes, static_cast<long long>(e_local) * n, k / 2, kBlockF);
-    if (rc == DLM_OK) rc = make_map_u8(&w->tm_a, rows, static_cast<long long>(e_local) * m_max, k / 2, 8);
-    w->w_scales = static_cast<const uint8_t*>(scales), w->a_scales = static_cast<const uint8_t*>(row_scales);
-    w->alpha = alpha, w->n = n, w->k = k;
-    return rc;
-}
-
-// The down-projection and the combine.
 static int fill_moe(MoeDev* d, const DlmMoe* m) {
     std::memset(d, 0, sizeof(*d));
-    const int rc = fill_gemm_half(&d->gemm[1], m->w_codes, m->w_tiled, m->w_scales, m->act_codes, m->act_scales, m->g2,
-                                  m->e_local, m->m_max, m->n, m->f);
+    int rc = DLM_OK;
+    if (m->w_tiled) d->w_tiles = static_cast<const uint8_t*>(m->w_codes);
+    else rc = make_map_u8(&d->tm_w, m->w_codes, static_cast<long long>(m->e_local) * m->n, m->f / 2, kBlockF);
+    if (rc == DLM_OK) rc = make_map_u8(&d->tm_a, m->act_codes, static_cast<long long>(m->e_local) * m->m_max, m->f / 2, 8);
     if (rc != DLM_OK) return rc;
-    d->amap = m->amap, d->counts = m->counts, d->ids = m->ids, d->weights = m->weights;
+    d->a_scales = static_cast<const uint8_t*>(m->act_scales);
+    d->w_scales = static_cast<const uint8_t*>(m->w_scales);
+    d->amap = m->amap, d->counts = m->counts, d->g2 = m->g2, d->ids = m->ids, d->weights = m->weights;
     d->shared = static_cast<const __nv_bfloat16*>(m->shared);
     d->gen = static_cast<int*>(m->workspace);
     d->counters = d->gen + kEpochSlots;
-    d->y = reinterpret_cast<__nv_bfloat16*>(static_cast<char*>(m->workspace) + kMoeWorkspaceHeader);
-    d->m = m->m, d->top_k = m->top_k, d->m_max = m->m_max;
+    d->y = reinterpret_cast<__nv_bfloat16*>(static_cast<char*>(m->workspace) + kWorkspaceHeader);
+    d->m = m->m, d->n = m->n, d->f = m->f, d->top_k = m->top_k, d->m_max = m->m_max;
     d->lo = m->lo, d->e_local = m->e_local, d->e_total = m->e_total;
     set_layout(d);
     return DLM_OK;
 }
 
-// What the combine alone needs to know.
-static void fill_combine(MoeDev* d, const DlmMoe* m) {
-    d->gemm[1].n = m->n, d->gemm[1].k = m->f;
-    d->ids = m->ids, d->weights = m->weights;
-    d->shared = static_cast<const __nv_bfloat16*>(m->shared);
-    d->y = reinterpret_cast<__nv_bfloat16*>(static_cast<char*>(m->workspace) + kMoeWorkspaceHeader);
-    d->m = m->m, d->top_k = m->top_k, d->lo = m->lo, d->e_local = m->e_local, d->e_total = m->e_total;
-}
-
 size_t dlm_moe_workspace_bytes(int m, int n, int top_k) {
     if (m <= 0 || n <= 0 || top_k <= 0) return 0;
-    return kMoeWorkspaceHeader + static_cast<size_t>(m) * top_k * n * 2;
+    return kWorkspaceHeader + static_cast<size_t>(m) * top_k * n * 2;
 }
 
 int dlm_moe_nvfp4(const DlmMoe* moe, void* out, int64_t ldo, int pdl, dlm_stream_t stream) {
@@ -627,11 +608,11 @@ static int check_front(const DlmMoeFront* a) {
     return DLM_OK;
 }
 
-// The whole call up to the experts' outputs in `moe`'s workspace, or without `moe` up to the down-projection's input:
-// two launches, the bookkeeping + quantisation and the GEMM(s).
-static int run_routed(const DlmMoeFront* a, const DlmMoe* moe, int pdl, dlm_stream_t stream) {
+int dlm_moe_front_nvfp4(const DlmMoeFront* a, int pdl, dlm_stream_t stream) {
+    int rc = check_front(a);
+    if (rc != DLM_OK) return rc;
     DeviceInfo info;
-    int rc = device_info(&info);
+    rc = device_info(&info);
     if (rc != DLM_OK) return rc;
     PrepareDev prep;
     std::memset(&prep, 0, sizeof(prep));
@@ -642,79 +623,28 @@ static int run_routed(const DlmMoeFront* a, const DlmMoe* moe, int pdl, dlm_stre
     prep.slot_codes = static_cast<uint8_t*>(a->slot_codes), prep.slot_scales = static_cast<uint8_t*>(a->slot_scales);
     prep.rows = a->m, prep.hidden = a->hidden, prep.top_k = a->top_k, prep.e_total = a->e_total;
     prep.lo = a->lo, prep.e_local = a->e_local, prep.m_max = a->m_max;
-    MoeParams<1> p;
-    std::memset(&p, 0, sizeof(p));
-    MoeDev* d = &p.g[0];
-    if (moe != nullptr) {
-        rc = fill_moe(d, moe);
-        if (rc != DLM_OK) return rc;
-        d->gen = reinterpret_cast<int*>(static_cast<char*>(moe->workspace) + kWorkspaceHeader);
-        d->done = d->gen + kEpochSlots;
-    } else {
-        d->m = a->m, d->top_k = a->top_k, d->m_max = a->m_max;
-        d->lo = a->lo, d->e_local = a->e_local, d->e_total = a->e_total;
-        d->gemm[1].k = a->f;
-    }
-    // Gate / up: the "output features" are the 2F interleaved rows, K is the hidden size.
-    rc = fill_gemm_half(&d->gemm[0], a->w13_codes, a->w13_tiled, a->w13_scales, a->slot_codes, a->slot_scales, a->g1,
-                        a->e_local, a->m_max, 2 * a->f, a->hidden);
-    if (rc != DLM_OK) return rc;
-    d->packed = a->packed, d->amap = a->amap, d->counts = a->counts;
-    d->a2_inv = a->a2_inv, d->act_kind = a->activation;
-    d->aq_out = static_cast<uint8_t*>(a->act_codes), d->as_out = static_cast<uint8_t*>(a->act_scales);
-    set_layout(d);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     rc = launch_moe_prepare(prep, {s, pdl != 0, false});
     if (rc != DLM_OK) return rc;
-    return launch_moe_whole(p, info.sms, {s, true, false});  // always a dependent launch of the kernel above
-}
-
-int dlm_moe_front_nvfp4(const DlmMoeFront* a, int pdl, dlm_stream_t stream) {
-    const int rc = check_front(a);
-    return rc != DLM_OK ? rc : run_routed(a, nullptr, pdl, stream);
-}
-
-int dlm_moe_experts_nvfp4(const DlmMoeFront* a, const DlmMoe* moe, int pdl, dlm_stream_t stream) {
-    int rc = check_front(a);
-    if (rc == DLM_OK) rc = check_moe(moe);
-    if (rc != DLM_OK) return rc;
-    if (moe->m != a->m || moe->n != a->hidden || moe->f != a->f || moe->top_k != a->top_k || moe->m_max != a->m_max ||
-        moe->lo != a->lo || moe->e_local != a->e_local || moe->e_total != a->e_total || moe->act_codes != a->act_codes ||
-        moe->act_scales != a->act_scales)
-        return DLM_ERR_SHAPE;
-    return run_routed(a, moe, pdl, stream);
-}
-
-int dlm_moe_combine(const DlmMoe* moe, void* out, int64_t ldo, int pdl, dlm_stream_t stream) {
-    int rc = check_moe(moe);
-    if (rc != DLM_OK) return rc;
-    if (out == nullptr) return DLM_ERR_NULL;
-    if (!aligned16(out) || ldo < moe->n || ldo % 8) return DLM_ERR_ALIGN;
+    // GEMM1 on the expert pipeline: the "output features" are the 2F interleaved gate / up rows, K is the hidden size.
     MoeParams<1> p;
     std::memset(&p, 0, sizeof(p));
-    fill_combine(&p.g[0], moe);
-    p.g[0].out = static_cast<__nv_bfloat16*>(out);
-    p.g[0].ldo = ldo;
-    return launch_combine(p, moe->m, {static_cast<cudaStream_t>(stream), pdl != 0, false});
-}
-
-int dlm_rowpar_moe_combine(const DlmMoe* moe, const DlmComm* comm, dlm_stream_t stream) {
-    int rc = check_moe(moe);
-    if (rc == DLM_OK) rc = check_comm(comm);
+    MoeDev* d = &p.g[0];
+    if (a->w13_tiled) d->w_tiles = static_cast<const uint8_t*>(a->w13_codes);
+    else rc = make_map_u8(&d->tm_w, a->w13_codes, static_cast<long long>(a->e_local) * 2 * a->f, a->hidden / 2, kBlockF);
+    if (rc == DLM_OK)
+        rc = make_map_u8(&d->tm_a, a->slot_codes, static_cast<long long>(a->e_local) * a->m_max, a->hidden / 2, 8);
     if (rc != DLM_OK) return rc;
-    if (moe->m != comm->rows || moe->n != comm->n) return DLM_ERR_SHAPE;
-    DeviceInfo info;
-    rc = device_info(&info);
-    if (rc != DLM_OK) return rc;
-    MoeParams<1> p;
-    std::memset(&p, 0, sizeof(p));
-    fill_combine(&p.g[0], moe);
-    fill_comm(&p.c[0], comm);
-    p.fused = 1;
-    int grid = comm->max_ctas > 0 && comm->max_ctas < info.sms ? comm->max_ctas : info.sms;
-    // One rank: blocks wait for nobody, so one block per row, unless the caller caps the grid.
-    if (comm->world == 1 && (grid > moe->m || (comm->max_ctas == 0 && comm->stamps == nullptr))) grid = moe->m;
-    return launch_combine(p, grid, {static_cast<cudaStream_t>(stream), comm->pdl != 0, false});
+    d->a_scales = static_cast<const uint8_t*>(a->slot_scales);
+    d->w_scales = static_cast<const uint8_t*>(a->w13_scales);
+    d->amap = a->amap, d->counts = a->counts, d->g2 = a->g1, d->a2_inv = a->a2_inv;
+    d->aq_out = static_cast<uint8_t*>(a->act_codes), d->as_out = static_cast<uint8_t*>(a->act_scales);
+    d->m = a->m, d->n = 2 * a->f, d->f = a->hidden, d->top_k = a->top_k, d->m_max = a->m_max;
+    d->lo = a->lo, d->e_local = a->e_local, d->e_total = a->e_total;
+    d->f_out = a->f, d->act_kind = a->activation;
+    set_layout(d);
+    p.fused = 0;
+    return launch_moe_gate_up(p, info.sms, {s, true, false});  // always a dependent launch of the kernel above
 }
 
 int dlm_route_packed(const void* logits, const void* scale, int32_t* packed, int rows, int e, int top_k, int pdl,

@@ -147,9 +147,6 @@ __device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xF
 __device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// Generic-proxy accesses before it, async-proxy accesses after it, in global memory as well.
-__device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
-
 // Asynchronous 4- and 16-byte global -> shared copies (no register staging) and their completion on an mbarrier:
 // the arrival fires once all of this thread's earlier cp.async copies have landed; .noinc means the barrier's
 // expected count must already include it.

@@ -44,44 +44,32 @@ struct alignas(64) RowparParams {
     int fused;  // 0: plain GEMM into g.out; 1: push + reduce
 };
 
-constexpr int kMaxEntries = 512;    // (expert, block of rows) pairs of one expert launch
-// Behind the header of an expert workspace: the whole call's launch generation [256] and entry counters [2][kMaxEntries].
-constexpr int kMoeWorkspaceHeader = kWorkspaceHeader + (kEpochSlots + 2 * kMaxEntries) * 4;
-
-// One of the experts' two GEMMs: n output rows (2F interleaved gate / up rows, or the hidden size), k inputs.
-struct alignas(64) ExpertGemm {
-    CUtensorMap tm_w;         // weight codes as bytes [e_local * n, k / 2], box 128 B x 128 rows, 128-byte swizzle
-    CUtensorMap tm_a;         // activation codes [e_local * m_max, k / 2], box 128 B x 8 rows, 128-byte swizzle
-    const uint8_t* w_tiles;   // or: the codes pre-tiled [e_local][n / 128][ceil(k / 256)][16 KB], each tile 128 rows x 128
-                              // bytes already in the swizzled shared-memory order (zero-padded along k)
-    const uint8_t* w_scales;  // [e_local][n / 128][k / 64][512] E4M3 in 128 x 4 atoms
-    const uint8_t* a_scales;  // [e_local * m_max, k / 16] E4M3, linear
-    const float* alpha;       // [e_local] input scale x weight scale
-    int n, k;                 // n = 0: the launch has no such GEMM
-};
-
-// The NVFP4 routed experts of one rank: gate / up (gemm[0]; whole calls only), down-projection (gemm[1]) + combine.
+// The NVFP4 expert down-projection of one rank (GEMM2 of the routed experts + the weighted combine).
 struct alignas(64) MoeDev {
-    ExpertGemm gemm[2];
-    const int* packed;        // whole call: [m, top_k] expert << 16 | BF16 weight bits
+    CUtensorMap tm_w;         // W2 codes as bytes [e_local * n, f / 2], box 128 B x 128 rows, 128-byte swizzle
+    const uint8_t* w_tiles;   // or: the codes pre-tiled [e_local][n / 128][ceil(f / 256)][16 KB], each tile 128 rows x 128
+                              // bytes already in the swizzled shared-memory order (zero-padded along f)
+    CUtensorMap tm_a;         // activation codes [e_local * m_max, f / 2], box 128 B x 8 rows, 128-byte swizzle
+    const uint8_t* a_scales;  // [e_local * m_max, f / 16] E4M3, linear
+    const uint8_t* w_scales;  // [e_local][n / 128][f / 64][512] E4M3 in 128 x 4 atoms
     const int* amap;          // [e_total, m_max] pair index (token * top_k + k) of each expert's slots
     const int* counts;        // [e_total]
+    const float* g2;          // [e_local]
     const int* ids;           // [m, top_k] global expert ids
     const float* weights;     // [m, top_k]
-    const __nv_bfloat16* shared;  // [m, hidden] or null
-    __nv_bfloat16* y;         // [m * top_k, hidden] per-(token, expert) outputs (workspace)
-    int* gen;                 // workspace: launch generation [256] (of the whole call or of the down-projection alone)
-    int* counters;            //            arrival counters [2][kMaxTiles] of the down-projection alone
-    int* done;                //            entry counters [2][kMaxEntries] of the whole call
-    __nv_bfloat16* out;       // plain (unfused) output [m, hidden]
+    const __nv_bfloat16* shared;  // [m, n] or null
+    __nv_bfloat16* y;         // [m * top_k, n] per-(token, expert) outputs (workspace)
+    int* gen;                 // workspace header: launch generation [256]
+    int* counters;            //                   arrival counters [2][kMaxTiles]
+    __nv_bfloat16* out;       // plain (unfused) output [m, n]
     long long ldo;
-    int m, top_k, m_max, lo, e_local, e_total;
+    int m, n, f, top_k, m_max, lo, e_local, e_total;
     int stages, rows_cap, buffers;  // shared memory: see moe_layout
-    // gate / up only
+    // GEMM1 (gate / up) only: n = 2F interleaved weight rows, f = hidden, g2 = the GEMM1 alpha g1
     const float* a2_inv;      // [e_local] 1 / (GEMM2 input scale): global scale of the activation's NVFP4 rounding
-    uint8_t* aq_out;          // [e_local * m_max, F / 2] activation codes written into the expert-major slots
-    uint8_t* as_out;          // [e_local * m_max, F / 16] their E4M3 scales (linear)
-    int act_kind;             // 0 = SwiGLU, 1 = GeGLU (tanh GELU)
+    uint8_t* aq_out;          // [e_local * m_max, f_out / 2] activation codes written into the expert-major slots
+    uint8_t* as_out;          // [e_local * m_max, f_out / 16] their E4M3 scales (linear)
+    int f_out, act_kind;      // F; 0 = SwiGLU, 1 = GeGLU (tanh GELU)
 };
 
 // Routing bookkeeping + input quantisation in front of the experts' GEMM1 (one CTA per token).
@@ -130,8 +118,7 @@ int launch_rowpar(const RowparParams<1>& p, int grid, const LaunchOpts& o);
 int launch_rowpar_loopback(const RowparParams<kMaxWorld>& p, int grid, int nranks, const LaunchOpts& o);
 int launch_moe(const MoeParams<1>& p, int grid, const LaunchOpts& o);
 int launch_moe_loopback(const MoeParams<kMaxWorld>& p, int grid, int nranks, const LaunchOpts& o);
-int launch_moe_whole(const MoeParams<1>& p, int grid, const LaunchOpts& o);
-int launch_combine(const MoeParams<1>& p, int grid, const LaunchOpts& o);
+int launch_moe_gate_up(const MoeParams<1>& p, int grid, const LaunchOpts& o);
 int launch_moe_prepare(const PrepareDev& p, const LaunchOpts& o);
 int launch_route_packed(const RouteDev& p, const LaunchOpts& o);
 struct MoeLayout {

@@ -30,19 +30,13 @@
 // When all CTAs are through their items (arrival counter), rows of the output are combined from Y in FP32 and pushed
 // into the owner ranks' receive slots, and the reduction phases of comm.cuh follow.
 //
-// That is moe_kernel<NR, false>, for callers that hold the down-projection's input. A whole routed-expert call
-// (moe_kernel<1, true>) runs the same pipeline over two GEMMs in one launch: first the gate / up GEMM (the step in front
-// of the down-projection, dlmrt/ops/triton/nvfp4_moe.py:69-104 `_gate_up`), then the down-projection. W13 [2F x hidden]
-// streams with its rows interleaved (row 2i = gate feature i, row 2i + 1 = up feature i) so that a gate value and its up
-// value sit in neighbouring lanes of the accumulator; the entry's rows are the NVFP4-quantised tokens routed to it. The
-// epilogue scales by g1, applies SwiGLU or GeGLU in FP32, re-quantises to NVFP4 against 1 / a2 (per 16 features: E4M3
-// scale, E2M1 codes, the approximate-reciprocal recipe of nvfp4_moe.py:36-47) and writes codes and scales straight into
-// the expert-major slots the down-projection reads. An entry's down-projection waits until all its gate / up tiles have
-// been announced on the entry's counter; the weights of both GEMMs are one stream per CTA that never stops for it. In
-// two launches the stream stopped for 5-7 us in between (the slower CTAs of the first, launch, routing scan, the ring's
-// first fill). The list of entries is counted from the packed top-k itself, so the stream also starts while the kernel
-// that quantises and places the rows is still running. This form ends with Y; combine_kernel, launched by the reduction
-// (or at once, where there is none), does the rest.
+// The same pipeline, instantiated with GATE_UP, is GEMM1 of the experts (the step in front of the down-projection,
+// dlmrt/ops/triton/nvfp4_moe.py:69-104 `_gate_up`): W13 [2F x hidden] streams instead of W2, its rows interleaved
+// (row 2i = gate feature i, row 2i + 1 = up feature i) so that a gate value and its up value sit in neighbouring lanes
+// of the accumulator; the expert's rows are the NVFP4-quantised tokens routed to it. The epilogue scales by g1, applies
+// SwiGLU or GeGLU in FP32, re-quantises to NVFP4 against 1 / a2 (per 16 features: E4M3 scale, E2M1 codes, the
+// approximate-reciprocal recipe of nvfp4_moe.py:36-47) and writes codes and scales straight into the expert-major
+// slots the down-projection reads. It ends there: no combine, no reduction.
 #include "kernels.cuh"
 
 namespace dlm {
@@ -62,7 +56,7 @@ constexpr int kMaxRowsCap = 128;       // rows of one entry: the MMA's N
 constexpr int kTmemAcc = 0, kTmemSfa = 256, kTmemSfb = 288, kTmemCols = 512;
 constexpr int kSfbSteps = (kTmemCols - kTmemSfb) / 4;
 constexpr int kMaxLocalExperts = 256;
-static_assert(kMaxEntries >= kMaxLocalExperts + 256 * 16 / 16, "one entry per active expert + one per 16 of 4096 pairs");
+constexpr int kMaxEntries = 2 * kMaxLocalExperts;  // one per active expert + one per 16 rows of 4096 pairs at most
 constexpr int kMoeStages = 12;
 constexpr int kMoeSmemBudget = 222 * 1024;
 
@@ -76,7 +70,6 @@ struct MoeSmem {
     uint32_t tmem_base;
     int n_active, epoch, gen, failed;
     int warp_count[8];
-    int counted[kMaxLocalExperts];  // whole call: rows of each expert, counted from the packed top-k
     float scratch[64];
     short active[kMaxEntries];  // expert | row block << 8
     short rows[kMaxEntries];    // rows of that block
@@ -119,8 +112,7 @@ MoeLayout moe_layout(int k, int m_max, int mean_rows) {
 }
 
 static int moe_smem_bytes(const MoeDev& d) {
-    const int k = d.gemm[0].n > 0 && d.gemm[0].k > d.gemm[1].k ? d.gemm[0].k : d.gemm[1].k;
-    return d.stages * kStageBytes + d.buffers * entry_bytes(d.rows_cap, k) + static_cast<int>(sizeof(MoeSmem)) + 1024;
+    return d.stages * kStageBytes + d.buffers * entry_bytes(d.rows_cap, d.f) + static_cast<int>(sizeof(MoeSmem)) + 1024;
 }
 
 // A token's expert list for the combine step, eight entries at a time: local expert index (or -1) and routing weight.
@@ -157,7 +149,7 @@ __device__ __forceinline__ uint4 combine_row(const MoeDev& g, int row, int t, co
         for (int j = 0; j < kCombineBatch; ++j) {
             raw[j] = make_uint4(0, 0, 0, 0);
             if (m.e[j] >= 0)
-                raw[j] = __ldcg(reinterpret_cast<const uint4*>(g.y + static_cast<size_t>(row * g.top_k + k0 + j) * g.gemm[1].n) + t);
+                raw[j] = __ldcg(reinterpret_cast<const uint4*>(g.y + static_cast<size_t>(row * g.top_k + k0 + j) * g.n) + t);
         }
 #pragma unroll
         for (int j = 0; j < kCombineBatch; ++j) {
@@ -177,7 +169,7 @@ __device__ __forceinline__ uint4 combine_row(const MoeDev& g, int row, int t, co
     if (g.shared) {
         float v[kVec] = {};
         add_bf16x8(v, packed);
-        add_bf16x8(v, *(reinterpret_cast<const uint4*>(g.shared + static_cast<size_t>(row) * g.gemm[1].n) + t));
+        add_bf16x8(v, *(reinterpret_cast<const uint4*>(g.shared + static_cast<size_t>(row) * g.n) + t));
         packed = pack_bf16x8(v);
     }
     return packed;
@@ -187,7 +179,7 @@ __device__ __forceinline__ uint4 combine_row(const MoeDev& g, int row, int t, co
 template <int MODE>
 __device__ __forceinline__ void combine_and_finish(const MoeDev& g, const CommDev& c, int block, int blocks, float* scratch,
                                                    const CombineMeta& first) {
-    const int t = threadIdx.x, threads = g.gemm[1].n / kVec;
+    const int t = threadIdx.x, threads = g.n / kVec;
     const bool active = t < threads;
     const int col = (active ? t : 0) * kVec;
     uint4 wraw = make_uint4(0, 0, 0, 0);
@@ -201,44 +193,6 @@ __device__ __forceinline__ void combine_and_finish(const MoeDev& g, const CommDe
             add_bf16x8(v, combine_row(g, row, t, row == block ? first : combine_meta(g, row, 0)));
         }
         finish_row<MODE>(c, v, hraw, wraw, off, active, true, scratch, threads);
-    }
-}
-
-// Combine: out[row] = bf16(sum over k in list order of w_k * y_k), experts of other ranks contribute 0 * 0; then, fused,
-// the reduction over ranks. With one rank the sum over ranks is the identity and the CTA that combines a row is also its
-// owner (rows block, block + blocks, ... in both roles), so the row is finished here and never travels through the receive
-// slots. `first`: the expert list of row `block`, fetched before the wait for Y.
-__device__ __forceinline__ void combine_tail(const MoeDev& g, const CommDev& c, bool fused, const CommCtx& x, int block,
-                                             int blocks, float* scratch, const CombineMeta& first) {
-    const bool local_rows = fused && c.world == 1;
-    if (local_rows) {
-        if (x.dead) return;
-        if (c.mode == kReduce) combine_and_finish<kReduce>(g, c, block, blocks, scratch, first);
-        else if (c.mode == kReduceNorm) combine_and_finish<kReduceNorm>(g, c, block, blocks, scratch, first);
-        else combine_and_finish<kReduceNormResidual>(g, c, block, blocks, scratch, first);
-    } else {
-        const int t = threadIdx.x, threads = g.gemm[1].n / kVec;
-        for (int row = block; row < g.m; row += blocks) {
-            if (t < threads) {
-                const uint4 packed = combine_row(g, row, t, row == block ? first : combine_meta(g, row, 0));
-                if (fused) {
-                    push_store(c, x, row, t * kVec, packed);
-                } else {
-                    store_v4(g.out + static_cast<size_t>(row) * g.ldo + t * kVec, packed);
-                }
-            }
-        }
-    }
-    if (fused) {
-        stamp(c, x, 1);
-        if (local_rows) {  // no slot was written: nothing to re-arm, the invocation counters stay where they are
-            stamp(c, x, 2);
-            stamp(c, x, 3);
-        } else {
-            rearm_early(c, x);
-            own_and_collect(c, x, scratch);  // re-arms late shares between its own and collect phases
-            comm_end(c, x);
-        }
     }
 }
 
@@ -308,7 +262,7 @@ __device__ __forceinline__ void requantise_chunk(const MoeDev& g, const uint32_t
     const uint32_t sf = f32_to_e4m3(a2i * (amax * rcp_approx(6.f)));
     const float scale = amax != 0.f ? rcp_approx(e4m3_to_f32(sf) * rcp_approx(a2i)) : 0.f;
     const int mine = (lane & 16 ? 4 : 0) + (lane & 8 ? 2 : 0) + (lane & 4 ? 1 : 0) + (odd ? 8 : 0);
-    const int groups = g.gemm[1].k / 16, half_f = g.gemm[1].k / 2;
+    const int groups = g.f_out / 16, half_f = g.f_out / 2;
     if (!(lane & 2) && mine < rows)
         g.as_out[static_cast<size_t>(slot + mine) * groups + ft * 4 + quarter] = static_cast<uint8_t>(sf);
     // Codes: the feature's neighbour (lane ^ 2) has the other nibble of each byte. The even feature's lane assembles the
@@ -328,7 +282,7 @@ __device__ __forceinline__ void requantise_chunk(const MoeDev& g, const uint32_t
     }
 }
 
-template <int NR, bool WHOLE>
+template <int NR, bool GATE_UP>
 __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_constant__ MoeParams<NR> p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const int slot = NR == 1 ? 0 : static_cast<int>(blockIdx.y);
@@ -338,12 +292,12 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
     const int block = static_cast<int>(blockIdx.x), blocks = static_cast<int>(gridDim.x);
     if (c.stamps && threadIdx.x == 0) c.stamps[block * kStampSlots + 7] = globaltimer();
 
-    // Phase 0 is the gate / up GEMM, phase 1 the down-projection; a launch may lack either (no output rows).
-    const int ft0 = WHOLE ? g.gemm[0].n / kBlockF : 0, ft1 = g.gemm[1].n / kBlockF;  // feature tiles
-    auto steps_of = [&](int ph) { return g.gemm[ph].k / 64; };  // K = 64 instructions per item
-    auto blocks_of = [&](int ph) { return (g.gemm[ph].k + 255) / 256; };
+    const int feature_tiles = g.n / kBlockF;
+    const int steps = g.f / 64;                  // K = 64 instructions per item
+    const int nkb = (steps + kStepsPerBlock - 1) / kStepsPerBlock;
+    const int scale_row = g.f / 16;              // bytes of scales per activation row
     const int row_tile = g.rows_cap * 128;       // bytes of one k-block of an entry's rows
-    const int rows_bytes = max(WHOLE ? entry_bytes(g.rows_cap, g.gemm[0].k) : 0, entry_bytes(g.rows_cap, g.gemm[1].k));
+    const int rows_bytes = entry_bytes(g.rows_cap, g.f);
 
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     // The ring's codes, then its scale atoms, then the entries' rows: everything the MMAs read swizzled is 1 KB aligned.
@@ -363,51 +317,25 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
             mbar_init(&sm->acc_empty[i], 4);  // one arrival per epilogue warp of the buffer's group
         }
         fence_barrier_init();
-        for (int ph = WHOLE ? 0 : 1; ph < 2; ++ph) {
-            if (g.gemm[ph].n == 0) continue;
-            if (!g.gemm[ph].w_tiles) tma_prefetch_descriptor(&g.gemm[ph].tm_w);
-            tma_prefetch_descriptor(&g.gemm[ph].tm_a);
-        }
+        if (!g.w_tiles) tma_prefetch_descriptor(&g.tm_w);
+        tma_prefetch_descriptor(&g.tm_a);
     }
     if (warp == 2) tmem_alloc(&sm->tmem_base, kTmemCols);
     // The next kernel of the stream may be set up from now on (its blocks move in as this kernel's blocks leave).
     pdl_launch_dependents();
-    if (WHOLE) {
-        // The kernel in front of this one (moe_prepare_kernel) lets this one start only after it has itself waited for
-        // everything before it, so the packed top-k can be read here already; what that kernel writes (the quantised
-        // rows in their slots, the slot map) is waited for by the roles that read it.
-        for (int e = threadIdx.x; e < kMaxLocalExperts; e += kMoeThreads) sm->counted[e] = 0;
-        __syncthreads();
-        const int pairs = g.m * g.top_k;
-        for (int base = threadIdx.x; base < pairs; base += 4 * kMoeThreads) {
-            int word[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int i = base + u * kMoeThreads;
-                word[u] = i < pairs ? __ldcg(g.packed + i) : -1;
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int e = (word[u] >> 16) - g.lo;
-                if (base + u * kMoeThreads < pairs && e >= 0 && e < g.e_local) atomicAdd(&sm->counted[e], 1);
-            }
-        }
-        __syncthreads();
-    } else {
-        // Routing (counts, slots, activations) comes from the previous kernels of the stream: nothing of it may be read
-        // before they are complete.
-        pdl_wait();
-    }
+    // Routing (counts, slots, activations) comes from the previous kernels of the stream: nothing of it may be read
+    // before they are complete.
+    pdl_wait();
     // Compact list of (expert, block of rows_cap rows) entries that have rows, in expert order.
     {
         const int e = threadIdx.x;
-        const int total_rows = e < g.e_local ? min(WHOLE ? sm->counted[e] : g.counts[g.lo + e], g.m_max) : 0;
+        const int total_rows = e < g.e_local ? min(g.counts[g.lo + e], g.m_max) : 0;
         int early = 0;  // the invocation counters, fetched in the same round trip as the counts
-        if (!WHOLE) {
+        if (!GATE_UP) {
             if (threadIdx.x == 352 && p.fused) early = c.epochs[block];
+            if (threadIdx.x == 353) early = g.gen[block];
             if (threadIdx.x == 354 && p.fused) early = comm_failed(c);
         }
-        if (threadIdx.x == 353 && g.gen != nullptr) early = g.gen[block];
         const int nb = (total_rows + g.rows_cap - 1) / g.rows_cap;
         int incl = nb;
 #pragma unroll
@@ -439,72 +367,46 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
     }
     if (c.stamps && threadIdx.x == 0) c.stamps[block * kStampSlots + 0] = globaltimer();
     const uint32_t tmem = uniform(sm->tmem_base);
-    const int entries = uniform(sm->n_active);
+    const int n_items = uniform(sm->n_active) * feature_tiles;
     const long long deadline = globaltimer() + (c.timeout_ns > 0 ? c.timeout_ns : kDefaultTimeoutNs);
 
-    // This CTA's runs of items: [begin0, end0) of phase 0 and [begin1, end1) of phase 1, an item being entry * feature
-    // tiles + tile. Phase 0 is dealt out evenly by items; phase 1 so that the k-blocks of both together are even (a CTA
-    // that got one item more of phase 0 gets fewer of phase 1), where phase 1 is long enough for that.
-    int begin0 = 0, end0 = 0, begin1, end1;
-    {
-        const int n0 = entries * ft0, n1 = entries * ft1;
-        auto share = [&](int n, int b) { return static_cast<int>(static_cast<long long>(n) * b / blocks); };
-        begin1 = share(n1, block), end1 = share(n1, block + 1);
-        if (WHOLE) {
-            begin0 = share(n0, block), end0 = share(n0, block + 1);
-            const int kb0 = blocks_of(0), kb1 = blocks_of(1);
-            const long long total = static_cast<long long>(n0) * kb0 + static_cast<long long>(n1) * kb1;
-            if (n1 > 0 && total >= static_cast<long long>(blocks) * ((n0 + blocks - 1) / blocks) * kb0) {
-                auto bound = [&](int b, int first0) {
-                    const long long left = total * b / blocks - static_cast<long long>(first0) * kb0;
-                    return min(n1, max(0, static_cast<int>((left + kb1 / 2) / kb1)));
-                };
-                begin1 = bound(block, begin0), end1 = block + 1 == blocks ? n1 : bound(block + 1, end0);
-            }
+    // This CTA's run of items, and its position in it: entry and feature tile advance together.
+    struct Cursor {
+        int entry, ft;
+        __device__ void next(int feature_tiles) {
+            if (++ft == feature_tiles) ft = 0, ++entry;
         }
-    }
-    const int items0 = end0 - begin0, items = items0 + max(0, end1 - begin1);
-    struct Item {
-        int ph, entry, ft;
     };
-    auto item_at = [&](int t) {  // the t-th item of this CTA, over both phases
-        Item at;
-        at.ph = WHOLE && t < items0 ? 0 : 1;
-        const int i = at.ph ? begin1 + t - items0 : begin0 + t, ft = at.ph ? ft1 : ft0;
-        at.entry = i / ft;
-        at.ft = i - at.entry * ft;
-        return at;
-    };
-    int* done = g.done;  // whole call: per entry, gate / up warp tiles written (this launch's bank)
-    if (WHOLE && done != nullptr) done += ((sm->gen + 1) & 1) * kMaxEntries;
+    const int i0 = static_cast<int>(static_cast<long long>(block) * n_items / blocks);
+    const int i1 = static_cast<int>(static_cast<long long>(block + 1) * n_items / blocks);
+    const int first_entry = i0 / feature_tiles;
+    const int last_entry = i1 > i0 ? (i1 - 1) / feature_tiles : first_entry - 1;
+    const Cursor start{first_entry, i0 - first_entry * feature_tiles};
 
     // Warps 0 to 2 run as whole warps on uniform values, one elected lane issuing (see uniform()).
     if (warp == 0) {
         const bool leader = elect_one();
         int st = 0;
         uint32_t phase = 1;  // waiting for parity 1 on a fresh barrier returns at once: the first lap is free
-        bool alive = true;
-        for (int t = 0; t < items && alive; ++t) {
-            const Item at = item_at(t);
-            const ExpertGemm& w = g.gemm[at.ph];
+        Cursor at = start;
+        for (int i = i0; i < i1; ++i, at.next(feature_tiles)) {
             const int e = uniform(sm->active[at.entry] & 0xFF);
-            const int nkb = blocks_of(at.ph), steps = steps_of(at.ph);
-            const size_t tile = static_cast<size_t>(e) * (at.ph ? ft1 : ft0) + at.ft;
-            const uint8_t* codes = w.w_tiles + tile * nkb * kCodeTileW;
-            const uint8_t* scales = w.w_scales + tile * steps * kAtom;
+            const size_t tile = static_cast<size_t>(e) * feature_tiles + at.ft;
+            const uint8_t* codes = g.w_tiles + tile * nkb * kCodeTileW;
+            const uint8_t* scales = g.w_scales + tile * steps * kAtom;
             for (int kb = 0; kb < nkb; ++kb) {
                 if (!mbar_wait_warp(&sm->empty[st], phase, deadline)) {
                     if (leader) report(c.status, kErrTimeout, st, kPhasePipeline, 0);
-                    alive = false;
+                    i = i1;
                     break;
                 }
                 const uint32_t scale_bytes = static_cast<uint32_t>(min(kStepsPerBlock, steps - kb * kStepsPerBlock)) * kAtom;
                 if (leader) {
                     mbar_expect_tx(&sm->full[st], kCodeTileW + scale_bytes);
-                    if (w.w_tiles)  // one contiguous 16 KB run of HBM, already in the swizzled shared-memory order
+                    if (g.w_tiles)  // one contiguous 16 KB run of HBM, already in the swizzled shared-memory order
                         bulk_load(tiles + st * kCodeTileW, codes + kb * kCodeTileW, kCodeTileW, &sm->full[st], kEvictFirst);
                     else
-                        tma_load_2d(tiles + st * kCodeTileW, &w.tm_w, &sm->full[st], kb * 128, e * w.n + at.ft * kBlockF,
+                        tma_load_2d(tiles + st * kCodeTileW, &g.tm_w, &sm->full[st], kb * 128, e * g.n + at.ft * kBlockF,
                                     kEvictFirst);
                     bulk_load(ring_scales + st * kStepsPerBlock * kAtom, scales + kb * kStepsPerBlock * kAtom, scale_bytes,
                               &sm->full[st], kEvictFirst);
@@ -514,82 +416,39 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
         }
         __syncwarp();
     } else if (warp == 2 || warp == 3) {
-        // The entries' rows: codes by TMA (warp 2, one lane), scales into the atoms (warp 3): atom byte
-        // (r % 32) * 16 + (r / 32) * 4 + j of step s holds scale 4 s + j of row r (< 128). A buffer is refilled once the
-        // MMAs of the entry it held have completed.
+        // The entries' rows: codes by TMA (warp 2, one thread), scales by asynchronous copies straight into the atoms
+        // (warp 3): atom byte (r % 32) * 16 + (r / 32) * 4 + j of step s holds scale 4 s + j of row r (< 128). A buffer is
+        // refilled once the MMAs of the entry it held have completed.
         const bool leader = elect_one();
-        if (WHOLE) pdl_wait();  // the slots are filled by the kernel in front
         int buf = 0;
         uint32_t phase = 1;
-        bool alive = true;
-        for (int ph = WHOLE ? 0 : 1; ph < 2 && alive; ++ph) {
-            const ExpertGemm& w = g.gemm[ph];
-            const int begin = ph ? begin1 : begin0, end = ph ? end1 : end0, ft = ph ? ft1 : ft0;
-            if (begin >= end) continue;
-            const int nkb = blocks_of(ph), steps = steps_of(ph), scale_row = w.k / 16;
-            for (int entry = begin / ft; entry <= (end - 1) / ft; ++entry) {
-                if (!mbar_wait_warp(&sm->a_empty[buf], phase, deadline)) {
-                    if (leader) report(c.status, kErrTimeout, buf, kPhasePipeline, 5);
-                    alive = false;
-                    break;
-                }
-                const int what = uniform(static_cast<int>(sm->active[entry])), cnt = uniform(static_cast<int>(sm->rows[entry]));
-                const int row0 = (what & 0xFF) * g.m_max + (what >> 8) * g.rows_cap;  // first slot of the entry
-                uint8_t* rows = entry_rows + buf * rows_bytes;
-                if (WHOLE && ph == 1) {
-                    // The entry's activations come out of phase 0 of this launch, from whichever CTAs had its tiles: four
-                    // warps announce each tile.
-                    bool ready = true;
-                    if (lane == 0) {
-                        int seen;
-                        while (true) {
-                            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(done + entry) : "memory");
-                            if (seen >= 4 * ft0) break;
-                            if (globaltimer() > deadline) {
-                                report(c.status, kErrTimeout, 0, kPhasePipeline, 7);
-                                ready = false;
-                                break;
-                            }
-                        }
-                    }
-                    if (!__all_sync(0xFFFFFFFFu, ready)) {
-                        alive = false;
-                        break;
-                    }
-                    fence_proxy_async_all();  // written through the generic proxy, read by TMA below
-                }
-                if (warp == 2) {
-                    const int boxes = (cnt + kBoxRows - 1) / kBoxRows;
-                    if (leader) {
-                        mbar_expect_tx(&sm->a_full[buf], static_cast<uint32_t>(nkb * boxes * kBoxRows * 128));
-                        for (int kb = 0; kb < nkb; ++kb)
-                            for (int b = 0; b < boxes; ++b)
-                                tma_load_2d(rows + kb * row_tile + b * kBoxRows * 128, &w.tm_a, &sm->a_full[buf], kb * 128,
-                                            row0 + b * kBoxRows, kEvictLast);
-                    }
-                } else {
-                    // Four rows' words in flight at a time. Not through L1, which may hold lines from before phase 0.
-                    uint8_t* atoms = rows + nkb * row_tile;
-                    const uint32_t* src = reinterpret_cast<const uint32_t*>(w.a_scales + static_cast<size_t>(row0) * scale_row);
-                    for (int r0 = 0; r0 < cnt; r0 += 4) {
-                        for (int s2 = lane; s2 < steps; s2 += 32) {
-                            uint32_t v[4];
-#pragma unroll
-                            for (int u = 0; u < 4; ++u)
-                                if (r0 + u < cnt) v[u] = __ldcg(src + static_cast<size_t>(r0 + u) * steps + s2);
-#pragma unroll
-                            for (int u = 0; u < 4; ++u) {
-                                const int r = r0 + u;
-                                if (r < cnt)
-                                    *reinterpret_cast<uint32_t*>(atoms + s2 * kAtom + (r % 32) * 16 + (r / 32) * 4) = v[u];
-                            }
-                        }
-                    }
-                    fence_proxy_async();  // written through the generic proxy, read by tcgen05.cp
-                    mbar_arrive(&sm->a_full[buf]);
-                }
-                if (++buf == g.buffers) buf = 0, phase ^= 1;
+        for (int entry = first_entry; entry <= last_entry; ++entry) {
+            if (!mbar_wait_warp(&sm->a_empty[buf], phase, deadline)) {
+                if (leader) report(c.status, kErrTimeout, buf, kPhasePipeline, 5);
+                break;
             }
+            const int what = uniform(static_cast<int>(sm->active[entry])), cnt = uniform(static_cast<int>(sm->rows[entry]));
+            const int row0 = (what & 0xFF) * g.m_max + (what >> 8) * g.rows_cap;  // first slot of the entry
+            uint8_t* rows = entry_rows + buf * rows_bytes;
+            if (warp == 2) {
+                const int boxes = (cnt + kBoxRows - 1) / kBoxRows;
+                if (leader) {
+                    mbar_expect_tx(&sm->a_full[buf], static_cast<uint32_t>(nkb * boxes * kBoxRows * 128));
+                    for (int kb = 0; kb < nkb; ++kb)
+                        for (int b = 0; b < boxes; ++b)
+                            tma_load_2d(rows + kb * row_tile + b * kBoxRows * 128, &g.tm_a, &sm->a_full[buf], kb * 128,
+                                        row0 + b * kBoxRows, kEvictLast);
+                }
+            } else {
+                uint8_t* atoms = rows + nkb * row_tile;
+                for (int r = 0; r < cnt; ++r) {
+                    const uint8_t* src = g.a_scales + static_cast<size_t>(row0 + r) * scale_row;
+                    uint8_t* dst = atoms + (r % 32) * 16 + (r / 32) * 4;
+                    for (int s2 = lane; s2 < steps; s2 += 32) cp_async_4(dst + s2 * kAtom, src + s2 * 4);
+                }
+                cp_async_arrive(&sm->a_full[buf]);
+            }
+            if (++buf == g.buffers) buf = 0, phase ^= 1;
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -601,17 +460,15 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
         auto operand = [&](uint32_t address) { return desc_hi | ((address & 0x3FFFF) >> 4); };
         auto atom = [&](uint32_t address) { return sf_hi | ((address & 0x3FFFF) >> 4); };
         const uint32_t ring = smem_u32(tiles), scales = smem_u32(ring_scales), rows0 = smem_u32(entry_rows);
+        const bool resident = steps <= kSfbSteps;  // the entry's row scales stay in tensor memory
         int st = 0, set = 0, buf = -1;
         uint32_t phase = 0, a_phase = 1;
         uint32_t rows = 0, idesc = 0;
         bool alive = true;
-        int last = -1;  // the entry (and phase) in the current buffer
-        for (int item = 0; item < items && alive; ++item) {
-            const Item at = item_at(item);
-            const int acc_buf = item & 1, nkb = blocks_of(at.ph), steps = steps_of(at.ph);
-            const bool resident = steps <= kSfbSteps;  // the entry's row scales stay in tensor memory
-            if (at.entry * 2 + at.ph != last) {  // a new entry
-                last = at.entry * 2 + at.ph;
+        Cursor at = start;
+        for (int i = i0; i < i1 && alive; ++i, at.next(feature_tiles)) {
+            const int item = i - i0, acc_buf = item & 1;
+            if (item == 0 || at.ft == 0) {  // a new entry
                 if (leader && buf >= 0) umma_commit(&sm->a_empty[buf]);
                 if (++buf == g.buffers) buf = 0;
                 if (buf == 0) a_phase ^= 1;
@@ -675,19 +532,18 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
         // group 1 the odd ones. What it needs from global memory (the expert's scale, the destination rows) changes with
         // the entry only.
         const int quarter = warp & 3, group = (warp - 4) >> 2;
-        int last = -1, cnt = 0, slot0 = 0;
-        float alpha = 0.f, a2i = 0.f;
+        int entry = -1, cnt = 0, slot0 = 0;
+        float g2 = 0.f, a2i = 0.f;
         int dest[kMaxRowsCap / 32];  // destination of row 32 q + lane
-        if (WHOLE) pdl_wait();  // the slot map is written by the kernel in front
-        for (int t = group; t < items; t += 2) {
-            const Item at = item_at(t);
-            const bool up = WHOLE && at.ph == 0;
-            if (at.entry * 2 + at.ph != last) {
-                last = at.entry * 2 + at.ph;
-                const int what = sm->active[at.entry], e = what & 0xFF, row0 = (what >> 8) * g.rows_cap;
-                cnt = sm->rows[at.entry];
-                alpha = g.gemm[at.ph].alpha[e];
-                if (up) {
+        Cursor at = start;
+        if (group == 1) at.next(feature_tiles);
+        for (int i = i0 + group; i < i1; i += 2, at.next(feature_tiles), at.next(feature_tiles)) {
+            if (at.entry != entry) {
+                entry = at.entry;
+                const int what = sm->active[entry], e = what & 0xFF, row0 = (what >> 8) * g.rows_cap;
+                cnt = sm->rows[entry];
+                g2 = g.g2[e];
+                if (GATE_UP) {
                     a2i = g.a2_inv[e];
                     slot0 = e * g.m_max + row0;
                 } else {
@@ -696,7 +552,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
                     for (int q = 0; q < kMaxRowsCap / 32; ++q) dest[q] = q * 32 + lane < cnt ? slots[q * 32 + lane] : -1;
                 }
             }
-            if (!mbar_wait(&sm->acc_full[group], (t >> 1) & 1, deadline)) {
+            if (!mbar_wait(&sm->acc_full[group], ((i - i0) >> 1) & 1, deadline)) {
                 report(c.status, kErrTimeout, 0, kPhasePipeline, 2);
                 break;
             }
@@ -709,29 +565,24 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
                 uint32_t r[16];
                 tmem_load_16(acc + chunk * 16, r);
                 tmem_load_wait();
-                if (up) {
-                    requantise_chunk(g, r, alpha, a2i, lane, cnt - chunk * 16, slot0 + chunk * 16, at.ft, quarter);
+                if (GATE_UP) {
+                    requantise_chunk(g, r, g2, a2i, lane, cnt - chunk * 16, slot0 + chunk * 16, at.ft, quarter);
                 } else {
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
                         const int pair = __shfl_sync(0xffffffff, dest[chunk / 2], (chunk & 1) * 16 + j);
                         if (pair >= 0)
-                            g.y[static_cast<size_t>(pair) * g.gemm[1].n + col] = __float2bfloat16_rn(__uint_as_float(r[j]) * alpha);
+                            g.y[static_cast<size_t>(pair) * g.n + col] = __float2bfloat16_rn(__uint_as_float(r[j]) * g2);
                     }
                 }
             }
             tcgen05_fence_before();
-            if (up && done != nullptr) fence_proxy_async_all();  // the slots are read by TMA, in this launch
             __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(&sm->acc_empty[group]);
-                if (up && done != nullptr) {
-                    __threadfence();
-                    atomicAdd(done + at.entry, 1);
-                }
-            }
+            if (lane == 0) mbar_arrive(&sm->acc_empty[group]);
         }
     }
+    // Every Y row this CTA produced is written; announce it and wait for the rest of the grid (the combine reads rows
+    // written by other CTAs). Counters are banked by launch generation as in the BF16 kernel.
     tcgen05_fence_before();
     __syncthreads();
     if (c.stamps && threadIdx.x == 0) c.stamps[block * kStampSlots + 4] = globaltimer();
@@ -739,18 +590,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
         tcgen05_fence_after();
         tmem_dealloc(tmem, kTmemCols);
     }
-    if (WHOLE) {  // Y is written: combine_kernel does the rest
-        if (g.gen != nullptr) {
-            const int gen = sm->gen + 1;
-            for (int i = block * kMoeThreads + threadIdx.x; i < kMaxEntries; i += blocks * kMoeThreads)
-                g.done[((gen + 1) & 1) * kMaxEntries + i] = 0;  // the bank the next launch counts in
-            if (threadIdx.x == 0)
-                for (int j = block; j < kEpochSlots; j += blocks) g.gen[j] = gen;
-        }
-        return;
-    }
-    // Every Y row this CTA produced is written; announce it and wait for the rest of the grid (the combine reads rows
-    // written by other CTAs). Counters are banked by launch generation as in the BF16 kernel.
+    if (GATE_UP) return;  // the activation slots are written; the down-projection launch that follows does the rest
     CommCtx x{};
     if (p.fused) x = comm_begin(c, block, blocks, sm->epoch, sm->failed);
     // The expert list of this CTA's first output row is fetched now, ahead of the wait for the experts' outputs.
@@ -780,26 +620,41 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
         __syncthreads();
     }
     if (c.stamps && threadIdx.x == 0) c.stamps[block * kStampSlots + 5] = globaltimer();
-    combine_tail(g, c, p.fused != 0, x, block, blocks, sm->scratch, first);
+    // Combine: out[row] = bf16(sum over k in list order of w_k * y_k), experts of other ranks contribute 0 * 0.
+    // With one rank the sum over ranks is the identity and the CTA that combines a row is also its owner (rows block,
+    // block + blocks, ... in both roles), so the row is finished here and never travels through the receive slots.
+    const bool local_rows = p.fused && c.world == 1;
+    if (local_rows) {
+        if (c.mode == kReduce) combine_and_finish<kReduce>(g, c, block, blocks, sm->scratch, first);
+        else if (c.mode == kReduceNorm) combine_and_finish<kReduceNorm>(g, c, block, blocks, sm->scratch, first);
+        else combine_and_finish<kReduceNormResidual>(g, c, block, blocks, sm->scratch, first);
+    } else {
+        const int t = threadIdx.x, threads = g.n / kVec;
+        for (int row = block; row < g.m; row += blocks) {
+            if (t < threads) {
+                const uint4 packed = combine_row(g, row, t, row == block ? first : combine_meta(g, row, 0));
+                if (p.fused) {
+                    push_store(c, x, row, t * kVec, packed);
+                } else {
+                    store_v4(g.out + static_cast<size_t>(row) * g.ldo + t * kVec, packed);
+                }
+            }
+        }
+    }
+    if (p.fused) {
+        stamp(c, x, 1);
+        if (local_rows) {  // no slot was written: nothing to re-arm, the invocation counters stay where they are
+            stamp(c, x, 2);
+            stamp(c, x, 3);
+        } else {
+            rearm_early(c, x);
+            own_and_collect(c, x, sm->scratch);  // re-arms late shares between its own and collect phases
+            comm_end(c, x);
+        }
+    }
 }
 
-// What follows a whole routed-expert call: the combine, and the reduction over ranks where there is one. With one rank
-// (or none) blocks wait for nobody, so the grid is one block per row.
-__global__ void __launch_bounds__(kFusedThreads, 1) combine_kernel(const __grid_constant__ MoeParams<1> p) {
-    __shared__ float scratch[64];
-    const MoeDev& g = p.g[0];
-    const CommDev& c = p.c[0];
-    const int block = static_cast<int>(blockIdx.x), blocks = static_cast<int>(gridDim.x);
-    pdl_launch_dependents();
-    pdl_wait();
-    CommCtx x{};
-    if (p.fused) x = comm_begin(c, block, blocks, c.world > 1 ? c.epochs[block] : 0, comm_failed(c));
-    CombineMeta first;
-    if (block < g.m) first = combine_meta(g, block, 0);
-    combine_tail(g, c, p.fused != 0, x, block, blocks, scratch, first);
-}
-
-template <int NR, bool WHOLE>
+template <int NR, bool GATE_UP>
 static int launch_impl(const MoeParams<NR>& p, dim3 grid, const LaunchOpts& o) {
     const int smem = moe_smem_bytes(p.g[0]);
     static bool raised[64] = {};
@@ -807,7 +662,7 @@ static int launch_impl(const MoeParams<NR>& p, dim3 grid, const LaunchOpts& o) {
     int dev = 0;
     (void)cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !raised[dev]) {
-        err = cudaFuncSetAttribute(moe_kernel<NR, WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        err = cudaFuncSetAttribute(moe_kernel<NR, GATE_UP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    kMoeSmemBudget + static_cast<int>(sizeof(MoeSmem)) + 1024);
         raised[dev] = err == cudaSuccess;
     }
@@ -831,7 +686,7 @@ static int launch_impl(const MoeParams<NR>& p, dim3 grid, const LaunchOpts& o) {
         }
         config.attrs = attrs;
         config.numAttrs = n;
-        err = cudaLaunchKernelEx(&config, moe_kernel<NR, WHOLE>, p);
+        err = cudaLaunchKernelEx(&config, moe_kernel<NR, GATE_UP>, p);
     }
     if (err != cudaSuccess) {
         g_last_cuda_error = static_cast<int>(err);
@@ -844,27 +699,7 @@ static int launch_impl(const MoeParams<NR>& p, dim3 grid, const LaunchOpts& o) {
 
 int launch_moe(const MoeParams<1>& p, int grid, const LaunchOpts& o) { return launch_impl<1, false>(p, dim3(grid), o); }
 
-int launch_moe_whole(const MoeParams<1>& p, int grid, const LaunchOpts& o) { return launch_impl<1, true>(p, dim3(grid), o); }
-
-int launch_combine(const MoeParams<1>& p, int grid, const LaunchOpts& o) {
-    cudaLaunchConfig_t config{};
-    config.gridDim = dim3(static_cast<unsigned>(grid));
-    config.blockDim = dim3(static_cast<unsigned>((p.g[0].gemm[1].n / kVec + 31) / 32 * 32));
-    config.stream = o.stream;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    config.attrs = &attr;
-    config.numAttrs = o.pdl ? 1 : 0;
-    const cudaError_t err = cudaLaunchKernelEx(&config, combine_kernel, p);
-    if (err != cudaSuccess) {
-        g_last_cuda_error = static_cast<int>(err);
-        (void)cudaGetLastError();
-        return -6;
-    }
-    ++g_launches;
-    return 0;
-}
+int launch_moe_gate_up(const MoeParams<1>& p, int grid, const LaunchOpts& o) { return launch_impl<1, true>(p, dim3(grid), o); }
 
 int launch_moe_loopback(const MoeParams<kMaxWorld>& p, int grid, int nranks, const LaunchOpts& o) {
     return launch_impl<kMaxWorld, false>(p, dim3(grid, nranks), o);

@@ -231,7 +231,9 @@ class Group:
         if kind == "linear":
             what.gemm(x, out)
         else:
-            what.run(out)
+            from ..quantization import nvfp4
+
+            nvfp4._run_down(what.m, out)
 
     def flush(self, partial):
         """Run a deferred producer on its own, for callers that read the partial before reducing it."""
@@ -337,7 +339,7 @@ class Group:
         if fusable and pending[0] == "linear":
             code = lib.dlm_rowpar_bf16(self._gemm(pending[1], pending[2], chain), comm, stream)
         elif fusable:  # the experts' down-projection + combine (+ shared) in front of the same reduction
-            code = pending[1].reduce(comm, stream)
+            code = lib.dlm_rowpar_nvfp4_moe(pending[1].m, comm, stream)
         else:
             if pending is not None:
                 self._run_alone(pending)

@@ -161,7 +161,7 @@ def moe_down(act_codes, act_scales, amap, counts, experts, ids, weights, buffers
     `replicated`: every rank holds and updates the whole residual stream (LLaDA2), see `Group.reduce_norm`."""
     m = descriptor(act_codes, act_scales, amap, counts, experts, ids, weights, buffers, num_experts, shared)
     if group is None:
-        return Down(m).run(out)
+        return _run_down(m, out)
     stream = _lib.stream(act_codes)
     mode = _lib.REDUCE if norm_weight is None else _lib.REDUCE_NORM_RESIDUAL if h is not None else _lib.REDUCE_NORM
     comm, reduced = group._comm(m.m, m.n, site, chain, mode, h, norm_weight, eps, scale, replicated and h is not None)
@@ -173,25 +173,19 @@ def moe_down(act_codes, act_scales, amap, counts, experts, ids, weights, buffers
 ACTIVATIONS = {"swiglu": 0, "geglu": 1}
 
 
+def _run_down(m, out):
+    """The down-projection + combine described by `m`, without a reduction behind it."""
+    code = _lib.lib().dlm_moe_nvfp4(m, out.data_ptr(), out.stride(0), 1, _lib.stream(out))
+    if code:
+        _lib.check(code, "moe_down")
+    return out
+
+
 class Down:
-    """What is left of an expert call until the reduction of its output: the descriptor, the tensors it points to, and
-    whether the down-projection has run (then only the combine is left)."""
+    """A down-projection put off until the reduction of its output: the descriptor, and the tensors it points to."""
 
-    def __init__(self, m, *keep, combine_only=False):
-        self.m, self.keep, self.combine_only = m, keep, combine_only
-
-    def run(self, out):
-        """Finish the call without a reduction behind it."""
-        run = _lib.lib().dlm_moe_combine if self.combine_only else _lib.lib().dlm_moe_nvfp4
-        code = run(self.m, out.data_ptr(), out.stride(0), 1, _lib.stream(out))
-        if code:
-            _lib.check(code, "moe_down")
-        return out
-
-    def reduce(self, comm, stream):
-        """Finish it fused with the reduction `comm` describes; the library's return code."""
-        run = _lib.lib().dlm_rowpar_moe_combine if self.combine_only else _lib.lib().dlm_rowpar_nvfp4_moe
-        return run(self.m, comm, stream)
+    def __init__(self, m, *keep):
+        self.m, self.keep = m, keep
 
 
 class FrontBuffers:
@@ -246,8 +240,8 @@ def trtllm_moe(x, packed, experts, out, num_experts, lo, intermediate, quantized
     `shared` (not in the reference's signature): a BF16 [rows, hidden] addend folded into the combine, in place of the
     `torch.add(routed, shared, out=...)` that follows the call in dlmrt/models/llada2/model.py:360-362.
 
-    Three launches: per-token bookkeeping + input quantisation, both GEMMs (with the activation and its re-quantisation
-    between them), and the combine. When `out` is a symmetric partial of `experts["group"]`, the third is not run here but
+    Three launches: per-token bookkeeping + input quantisation, GEMM1 + activation + re-quantisation, and the
+    down-projection + combine. When `out` is a symmetric partial of `experts["group"]`, the third is not run here but
     deferred into the `Group.reduce*` of `out` that follows (one fused launch with the reduction over ranks)."""
     if quantized is None:
         rows, hidden = x.shape
@@ -277,16 +271,15 @@ def trtllm_moe(x, packed, experts, out, num_experts, lo, intermediate, quantized
     else:
         f.xq, f.xs = x.data_ptr(), xs.data_ptr()
     f.packed, f.top_k, f.activation = packed.data_ptr(), packed.shape[1], ACTIVATIONS[activation]
+    code = _lib.lib().dlm_moe_front_nvfp4(f, 1, _lib.stream(x))
+    if code:
+        _lib.check(code, "trtllm_moe: front half")
     m = DlmMoe.from_buffer_copy(b.back)
     m.shared = shared.data_ptr() if shared is not None else None
-    code = _lib.lib().dlm_moe_experts_nvfp4(f, m, 1, _lib.stream(x))
-    if code:
-        _lib.check(code, "trtllm_moe")
-    rest = Down(m, b, sources, shared, combine_only=True)
     group = experts.get("group")
     if group is not None and group.is_partial(out):
-        return group.defer_experts(out, rest)
-    return rest.run(out)
+        return group.defer_experts(out, Down(m, b, sources, shared))
+    return _run_down(m, out)
 
 
 def route_packed(logits, per_expert_scale, packed, top_k):

@@ -277,15 +277,6 @@ DLM_API size_t dlm_moe_workspace_bytes(int m, int n, int top_k);
  * (dlmrt/quantization/nvfp4.py:280-306). */
 DLM_API int dlm_moe_front_nvfp4(const DlmMoeFront* front, int pdl, dlm_stream_t stream);
 
-/* The whole of nvfp4.trtllm_moe up to the experts' outputs, which it leaves in moe->workspace: the bookkeeping +
- * quantisation, then ONE launch of both GEMMs (gate / up + activation + re-quantisation, down-projection), whose weights
- * are one uninterrupted stream. `moe` describes the down-projection of the same call: same sizes, and its act_codes /
- * act_scales are the front's. dlm_moe_combine (out[m, n] BF16) or dlm_rowpar_moe_combine (fused with the reduction over
- * ranks; moe->m == comm->rows, moe->n == comm->n) finishes the call: the weighted combine [+ shared]. */
-DLM_API int dlm_moe_experts_nvfp4(const DlmMoeFront* front, const DlmMoe* moe, int pdl, dlm_stream_t stream);
-DLM_API int dlm_moe_combine(const DlmMoe* moe, void* out, int64_t ldo, int pdl, dlm_stream_t stream);
-DLM_API int dlm_rowpar_moe_combine(const DlmMoe* moe, const DlmComm* comm, dlm_stream_t stream);
-
 /* The router's top-k as the reference packs it for this path (dlmrt/ops/triton/moe.py:70-73 `route_packed`): FP32
  * softmax of `logits` [rows, e] BF16, the top_k largest (ties to the lower expert), renormalised, times `scale` [e]
  * BF16, in ascending expert order, packed[rows, top_k] = expert << 16 | BF16 weight bits. e <= 256, top_k <= 16. */
