@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
     const int slot = NR == 1 ? 0 : static_cast<int>(blockIdx.y);
     const GemmDev& g = p.g[slot];
     const CommDev& c = p.c[slot];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
     const int block = static_cast<int>(blockIdx.x), blocks = static_cast<int>(gridDim.x);
     if (c.stamps && threadIdx.x == 0) c.stamps[block * kStampSlots + 7] = globaltimer();
 
@@ -185,8 +185,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
     const bool local_rows = p.fused && c.world == 1 && g.splits > 1;
 
     const int pre = iters < g.stages ? iters : g.stages;
+    // Warps 0, 1 and 3 run as whole warps on uniform values, one elected lane issuing (see uniform()).
+    const bool leader = elect_one();
     if (warp == 0) {
-        if (lane == 0) {
+        if (leader) {
             for (int i = 0; i < g.stages; ++i) {
                 mbar_init(&sm->full[i], 1);
                 mbar_init(&sm->empty[i], 1);
@@ -195,10 +197,12 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
             fence_barrier_init();
             if (!g.w_tiles) tma_prefetch_descriptor(&g.tm_w);
             tma_prefetch_descriptor(&g.tm_x);
-            // The first ring-full of loads is requested at once, by the thread that has just set the barriers up, while
-            // the rest of the block is still allocating tensor memory: weights depend on nothing, x only on the kernels
-            // in front of this one.
-            for (int it = 0; it < pre; ++it) {
+        }
+        // The first ring-full of loads is requested at once, by the thread that has just set the barriers up, while
+        // the rest of the block is still allocating tensor memory: weights depend on nothing, x only on the kernels
+        // in front of this one.
+        for (int it = 0; it < pre; ++it) {
+            if (leader) {
                 mbar_expect_tx(&sm->full[it], static_cast<uint32_t>(stage_bytes));
                 if (g.w_tiles)
                     bulk_load(tiles + it * stage_bytes, g.w_tiles + (static_cast<size_t>(f) * nkb + kb0 + it) * kTileBytesW,
@@ -207,30 +211,32 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
                     tma_load_2d(tiles + it * stage_bytes, &g.tm_w, &sm->full[it], (kb0 + it) * kBlockK, f * kBlockF,
                                 kEvictFirst);
             }
-            // The rest of this CTA's weight slab is pulled into L2 now: the ring then refills at L2 latency instead of
-            // HBM latency.
-            if (iters > pre && prefetch_rest_of_slab(mt)) {
-                if (g.w_tiles) {
-                    bulk_prefetch_l2(g.w_tiles + (static_cast<size_t>(f) * nkb + kb0 + pre) * kTileBytesW,
-                                     static_cast<uint32_t>(iters - pre) * kTileBytesW);
-                } else {
-                    for (int it = pre; it < iters; ++it) tma_prefetch_l2_2d(&g.tm_w, (kb0 + it) * kBlockK, f * kBlockF);
-                }
+        }
+        // The rest of this CTA's weight slab is pulled into L2 now: the ring then refills at L2 latency instead of
+        // HBM latency.
+        if (iters > pre && prefetch_rest_of_slab(mt) && leader) {
+            if (g.w_tiles) {
+                bulk_prefetch_l2(g.w_tiles + (static_cast<size_t>(f) * nkb + kb0 + pre) * kTileBytesW,
+                                 static_cast<uint32_t>(iters - pre) * kTileBytesW);
+            } else {
+                for (int it = pre; it < iters; ++it) tma_prefetch_l2_2d(&g.tm_w, (kb0 + it) * kBlockK, f * kBlockF);
             }
-            pdl_wait();
-            if (c.stamps) c.stamps[block * kStampSlots + 5] = globaltimer();
-            for (int it = 0; it < pre; ++it)
+        }
+        pdl_wait();
+        if (c.stamps && leader) c.stamps[block * kStampSlots + 5] = globaltimer();
+        for (int it = 0; it < pre; ++it) {
+            if (leader)
                 tma_load_2d(tiles + it * stage_bytes + kTileBytesW, &g.tm_x, &sm->full[it], (kb0 + it) * kBlockK,
                             token0, kEvictLast);
-            sm->seen[0] = sm->seen[1] = 0;
         }
-        __syncwarp();  // the warp reaches the block-wide barrier together
+        if (leader) sm->seen[0] = sm->seen[1] = 0;
+        __syncwarp();
     }
     if (warp == 2) tmem_alloc(&sm->tmem_base, cols * issuers);
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
-    const uint32_t tmem = sm->tmem_base;
+    const uint32_t tmem = uniform(sm->tmem_base);
     // The next kernel of the stream may be set up from now on: its blocks move in as this kernel's blocks leave, and it
     // waits for this kernel to complete before it reads anything this kernel writes.
     pdl_launch_dependents();
@@ -240,15 +246,15 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
     // 3 split-K rendezvous) and the k-block it was at.
     auto stalled = [](int who, int it) { return who << 24 | (it & 0xFFFF); };
     if (warp == 0) {
-        if (lane == 0) {
-            int st = pre == g.stages ? 0 : pre;
-            uint32_t parity = 0;  // second lap of the ring waits for the first release of each stage
-            for (int it = pre; it < iters; ++it) {
-                if (!mbar_wait(&sm->empty[st], parity, pipeline_deadline)) {
-                    report(c.status, kErrTimeout, st, kPhasePipeline, stalled(0, it));
-                    break;
-                }
-                uint8_t* stage = tiles + st * stage_bytes;
+        int st = pre == g.stages ? 0 : pre;
+        uint32_t parity = 0;  // second lap of the ring waits for the first release of each stage
+        for (int it = pre; it < iters; ++it) {
+            if (!mbar_wait_warp(&sm->empty[st], parity, pipeline_deadline)) {
+                if (leader) report(c.status, kErrTimeout, st, kPhasePipeline, stalled(0, it));
+                break;
+            }
+            uint8_t* stage = tiles + st * stage_bytes;
+            if (leader) {
                 mbar_expect_tx(&sm->full[st], static_cast<uint32_t>(stage_bytes));
                 if (g.w_tiles)
                     bulk_load(stage, g.w_tiles + (static_cast<size_t>(f) * nkb + kb0 + it) * kTileBytesW, kTileBytesW,
@@ -256,10 +262,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
                 else
                     tma_load_2d(stage, &g.tm_w, &sm->full[st], (kb0 + it) * kBlockK, f * kBlockF, kEvictFirst);
                 tma_load_2d(stage + kTileBytesW, &g.tm_x, &sm->full[st], (kb0 + it) * kBlockK, token0, kEvictLast);
-                if (++st == g.stages) st = 0, parity ^= 1;
             }
+            if (++st == g.stages) st = 0, parity ^= 1;
         }
-        __syncwarp();  // lanes 1-31 must not run ahead to the block-wide barrier while lane 0 is still issuing
+        __syncwarp();
     } else if (warp == 1 || warp == 3) {
         // MMA issue. One thread feeds the tensor pipe; for narrow tiles its own instruction stream (barrier wait,
         // descriptors, four MMAs, commit per k-block) is slower than the MMAs it issues, so tiles of up to 128 tokens
@@ -270,41 +276,44 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
         // sure the other one has seen k-block `it - stages` arrive (the same stage's previous phase): each publishes
         // the k-blocks it has seen in shared memory. The loads of `it` cannot have been requested before that anyway.
         const int who = warp == 1 ? 0 : 1;
-        if (lane == 0) {
-            if (who == 1) {
-                pdl_wait();
+        if (who == 1) {
+            pdl_wait();
+            if (leader) {
                 if (p.fused) sm->epoch = c.epochs[block], sm->failed = comm_failed(c);
                 if (g.splits > 1) sm->gen = g.gen[block];
             }
-            if (who < issuers) {
-                const uint32_t idesc = umma_idesc_bf16(kBlockF, mt);
-                const uint32_t acc = tmem + who * cols;
-                volatile int* seen = sm->seen;
-                const bool guarded = issuers == 2 && (g.stages & 1);  // see above; even rings need no hand-over
-                const uint64_t desc_hi = umma_desc_k128(tiles) & 0xFFFFFFFF00000000ull;
-                const uint32_t stage0 = smem_u32(tiles);
-                int st = 0;
-                uint32_t parity = 0;
-                for (int it = 0; it < iters; ++it) {
-                    if ((it & (issuers - 1)) == who) {
-                        bool ok = true;
-                        if (guarded && it >= g.stages) {  // k-block it - stages was the other issuer's
-                            while (seen[1 - who] <= it - g.stages) {
-                                if (globaltimer() > pipeline_deadline) {
-                                    ok = false;
-                                    break;
-                                }
+        }
+        if (who < issuers) {
+            const uint32_t idesc = umma_idesc_bf16(kBlockF, mt);
+            const uint32_t acc = tmem + who * cols;
+            volatile int* seen = sm->seen;
+            const bool guarded = issuers == 2 && (g.stages & 1);  // see above; even rings need no hand-over
+            const uint64_t desc_hi = umma_desc_k128(tiles) & 0xFFFFFFFF00000000ull;
+            const uint32_t stage0 = smem_u32(tiles);
+            int st = 0;
+            uint32_t parity = 0;
+            for (int it = 0; it < iters; ++it) {
+                if ((it & (issuers - 1)) == who) {
+                    bool ok = true;
+                    if (guarded && it >= g.stages) {  // k-block it - stages was the other issuer's
+                        while (seen[1 - who] <= it - g.stages) {
+                            if (globaltimer() > pipeline_deadline) {
+                                ok = false;
+                                break;
                             }
                         }
-                        if (!ok || !mbar_wait(&sm->full[st], parity, pipeline_deadline)) {
-                            report(c.status, kErrTimeout, st, kPhasePipeline, stalled(1, it));
-                            break;
-                        }
-                        if (guarded) seen[who] = it + 1;
-                        tcgen05_fence_after();
-                        const uint32_t base = stage0 + st * stage_bytes;
-                        const uint64_t dw = desc_hi | ((base & 0x3FFFF) >> 4);
-                        const uint64_t dx = desc_hi | (((base + kTileBytesW) & 0x3FFFF) >> 4);
+                        ok = __all_sync(0xFFFFFFFFu, ok);
+                    }
+                    if (!ok || !mbar_wait_warp(&sm->full[st], parity, pipeline_deadline)) {
+                        if (leader) report(c.status, kErrTimeout, st, kPhasePipeline, stalled(1, it));
+                        break;
+                    }
+                    if (guarded && leader) seen[who] = it + 1;
+                    tcgen05_fence_after();
+                    const uint32_t base = stage0 + st * stage_bytes;
+                    const uint64_t dw = desc_hi | ((base & 0x3FFFF) >> 4);
+                    const uint64_t dx = desc_hi | (((base + kTileBytesW) & 0x3FFFF) >> 4);
+                    if (leader) {
 #pragma unroll
                         for (int kk = 0; kk < kBlockK / kUmmaK; ++kk) {
                             // Advancing 16 BF16 = 32 bytes inside the swizzled row: +2 in the descriptor's 16-byte units.
@@ -312,10 +321,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
                         }
                         umma_commit(&sm->empty[st]);
                     }
-                    if (++st == g.stages) st = 0, parity ^= 1;
                 }
-                umma_commit(&sm->acc_full);
+                if (++st == g.stages) st = 0, parity ^= 1;
             }
+            if (leader) umma_commit(&sm->acc_full);
         }
         __syncwarp();
     } else if (warp >= 4) {
