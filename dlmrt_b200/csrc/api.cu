@@ -177,6 +177,39 @@ void choose_tiling(int m, int n, int k, int avail, int* tiles_out, int* splits_o
     }
 }
 
+// FP32 partial tiles of a GEMM whose K is split, as far as the library's own choice goes: kMaxSplits of every output tile,
+// or one tile of 128 features per SM where the output has so few that its K is split further.
+size_t partial_bytes(int m, int n) {
+    const size_t columns = static_cast<size_t>(kMaxSplits) * n, one_per_sm = static_cast<size_t>(148) * kBlockF;
+    return (columns > one_per_sm ? columns : one_per_sm) * m * sizeof(float);
+}
+
+// A plain GEMM of few output tiles and long K: kMaxSplits leave SMs idle (16 CTAs for 256 features), so choose_tiling's
+// pick is weighed against as many splits as there are SMs, half of them and so on. Beyond kMaxSplits every split costs
+// 0.2 us (the sum reads eight at a time, and fewer tokens are left for each CTA to sum). Measured, us with at most
+// kMaxSplits and beyond: 256 x 256 x 16384 14.3 and 11.8, 32 x 256 x 16384 13.5 and 10.0, 256 x 128 x 65536 40.5 and
+// 18.9; 64 x 512 x 4096 stays (7.7 with 8 splits, 7.9 with 9).
+void split_further(const DlmGemm* g, int avail, int* tiles, int* splits) {
+    const int feature_tiles = g->n / kBlockF, nkb = (g->k + kBlockK - 1) / kBlockK;
+    const double hbm = static_cast<double>(g->n) * g->k * 2 / 6.0e6;
+    auto cost = [&](int t, int sp) {
+        const int mt = g->m / t, kb = (nkb + sp - 1) / sp;
+        double us = kb * (0.24 + 0.0009 * mt);
+        if (us < hbm) us = hbm;
+        if (sp > 1) us += 2.8 + 0.019 * mt;
+        return us + (sp > kMaxSplits ? 0.2 * (sp - kMaxSplits) : 0);
+    };
+    const int64_t room = g->workspace_bytes - static_cast<int64_t>(kWorkspaceHeader), per_split = static_cast<int64_t>(g->m) * g->n * 4;
+    double best = cost(*tiles, *splits);
+    for (int t = 1; t <= 4 && g->m % (16 * t) == 0; t *= 2) {
+        for (int sp = avail / (feature_tiles * t); sp > kMaxSplits; sp /= 2) {
+            if (sp > nkb || sp * per_split > room) continue;
+            const double us = cost(t, sp);
+            if (us < best - 1e-9) best = us, *tiles = t, *splits = sp;
+        }
+    }
+}
+
 int check_gemm(const DlmGemm* g) {
     if (g == nullptr) return DLM_ERR_NULL;
     if (g->x == nullptr || g->w == nullptr || g->workspace == nullptr) return DLM_ERR_NULL;
@@ -194,7 +227,7 @@ int check_gemm(const DlmGemm* g) {
 
 // Fills the device-side GEMM block; returns the per-rank grid in *grid.
 int fill_gemm(GemmDev* d, const DlmGemm* g, int max_ctas, int sms, int* grid, int owner_rows = 0,
-              bool single_rank = false) {
+              bool single_rank = false, bool plain = false) {
     std::memset(d, 0, sizeof(*d));
     const int avail = max_ctas > 0 && max_ctas < sms ? max_ctas : sms;
     const int feature_tiles = g->n / kBlockF, nkb = (g->k + kBlockK - 1) / kBlockK;
@@ -203,6 +236,7 @@ int fill_gemm(GemmDev* d, const DlmGemm* g, int max_ctas, int sms, int* grid, in
         int t = 1, sp = 1;
         choose_tiling(g->m, g->n, g->k, avail, &t, &sp, owner_rows, single_rank);
         if (token_tiles == 0 && splits == 0) {
+            if (plain) split_further(g, avail, &t, &sp);
             token_tiles = t;
             splits = sp;
         } else if (token_tiles == 0) {
@@ -369,7 +403,7 @@ int dlm_gemm_bf16(const DlmGemm* gemm, void* out, int64_t ldo, int pdl, dlm_stre
     RowparParams<1> p;
     std::memset(&p, 0, sizeof(p));
     int grid = 0;
-    rc = fill_gemm(&p.g[0], gemm, 0, info.sms, &grid);
+    rc = fill_gemm(&p.g[0], gemm, 0, info.sms, &grid, 0, false, true);
     if (rc != DLM_OK) return rc;
     p.g[0].out = static_cast<__nv_bfloat16*>(out);
     p.g[0].ldo = ldo;
@@ -721,8 +755,7 @@ int dlm_rowpar_bf16_loopback(const DlmGemm* gemm, const DlmComm* comm, int nrank
 size_t dlm_workspace_bytes(int m, int n, int k) {
     (void)k;
     if (m <= 0 || n <= 0) return 0;
-    return kWorkspaceHeader +
-           static_cast<size_t>(kMaxSplits) * static_cast<size_t>(m) * static_cast<size_t>(n) * sizeof(float);
+    return kWorkspaceHeader + partial_bytes(m, n);
 }
 
 int dlm_choose_tiling(int m, int n, int k, int max_ctas, int* token_tiles, int* splits) {

@@ -11,7 +11,7 @@ constexpr int kFusedThreads = 384;  // 12 warps: TMA producer, MMA issuer, TMEM 
 constexpr int kBlockF = 128;        // weight rows (output features) per tile: the MMA's M
 constexpr int kBlockK = 64;         // BF16 per k-block: one 128-byte swizzled row
 constexpr int kUmmaK = 16;          // K of one tcgen05.mma kind::f16
-constexpr int kMaxSplits = 8;
+constexpr int kMaxSplits = 8;       // K splits a caller may ask for, and that a GEMM in front of a reduction takes
 constexpr int kMaxTiles = 128;      // (feature tiles) x (token tiles) of one GEMM
 constexpr int kWorkspaceHeader = 2048;  // int32 gen[256] then int32 counters[2][128]
 constexpr int kMaxStages = 8;

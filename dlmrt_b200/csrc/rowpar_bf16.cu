@@ -424,19 +424,20 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
         for (int v = threadIdx.x; v < (tok_hi - tok_lo) * (kBlockF / kVec); v += kFusedThreads) {
             const int token = tok_lo + v / (kBlockF / kVec), j = v % (kBlockF / kVec);
             const float* src = base + static_cast<size_t>(token) * kBlockF + j * kVec;
-            // Summed in split order, four splits' loads in flight at a time.
+            // Summed in split order, kBatch splits' loads in flight at a time.
+            constexpr int kBatch = 8;
             float acc[kVec];
-            for (int base_sp = 0; base_sp < g.splits; base_sp += 4) {
-                float4 a[4], b[4];
+            for (int base_sp = 0; base_sp < g.splits; base_sp += kBatch) {
+                float4 a[kBatch], b[kBatch];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
+                for (int u = 0; u < kBatch; ++u) {
                     if (base_sp + u < g.splits) {
                         a[u] = __ldcg(reinterpret_cast<const float4*>(src + (base_sp + u) * split_stride));
                         b[u] = __ldcg(reinterpret_cast<const float4*>(src + (base_sp + u) * split_stride) + 1);
                     }
                 }
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
+                for (int u = 0; u < kBatch; ++u) {
                     if (base_sp + u < g.splits) {
                         if (base_sp + u == 0) {
                             acc[0] = a[u].x, acc[1] = a[u].y, acc[2] = a[u].z, acc[3] = a[u].w;

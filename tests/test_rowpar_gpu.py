@@ -58,6 +58,30 @@ def test_gemm_exact_on_integer_operands(m, n, k):
     assert_same_bits(bits(gemm(x, w)), want, f"gemm {m}x{n}x{k}")
 
 
+@pytest.mark.parametrize("m, n, k", [(16, 128, 9472), (256, 128, 20040), (32, 256, 16384), (144, 384, 6408), (80, 640, 8200),
+                                     (64, 128, 640)])
+def test_gemm_of_few_tiles_splits_k_further(m, n, k):
+    """Outputs of one to five feature tiles: up to one split per SM, K ragged (20040, 6408, 8200 are no multiples of a
+    k-block), as many splits as k-blocks (640 = 10), tokens that do not divide among the splits. Twice on the same
+    workspace, whose counters alternate; and with no room beyond eight splits."""
+    from dlmrt_b200 import _lib
+    from dlmrt_b200._lib import DlmGemm
+
+    x, w = integer_case(m, n, k, seed=m + n + k)
+    want = f32_to_bf16(rowpar.gemm_f32(bits(x), bits(w)))
+    out = torch.empty(m, n, dtype=torch.bfloat16, device=x.device)
+    for nbytes in (_lib.lib().dlm_workspace_bytes(m, n, k), 2048 + 8 * m * n * 4):
+        ws = torch.zeros(nbytes, dtype=torch.uint8, device=x.device)
+        g = DlmGemm()
+        g.x, g.w, g.m, g.n, g.k, g.ldx, g.ldw = x.data_ptr(), w.data_ptr(), m, n, k, x.stride(0), w.stride(0)
+        g.workspace, g.workspace_bytes = ws.data_ptr(), ws.numel()
+        for _ in range(2):
+            out.fill_(-1)
+            _lib.check(_lib.lib().dlm_gemm_bf16(C.byref(g), out.data_ptr(), n, 0, None), "gemm")
+            torch.cuda.synchronize()
+            assert_same_bits(bits(out), want, f"gemm {m}x{n}x{k}, workspace {nbytes}")
+
+
 @pytest.mark.parametrize("m, n, k", SHAPES)
 def test_gemm_within_tolerance_on_gaussian_operands(m, n, k):
     """Tolerance of the GEMM partial: per row max-abs <= 2 BF16 ulp of the row's largest magnitude and relative L2
