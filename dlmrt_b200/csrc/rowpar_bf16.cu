@@ -51,11 +51,9 @@ __device__ __forceinline__ uint32_t tmem_cols(int m) {
 // announced its partial tile, sums the row's FP32 split partials in split order, rounds to BF16 (that is the rank's
 // partial, as the push path would have stored it) and finishes the row as any owner does. Thread t < n / 8 holds
 // columns [8t, 8t + 8): feature tile t / 16, 32 bytes of that tile's row. `scratch`: 64 floats.
-template <int MODE>
+template <int MODE, int kRows, int kGroup>
 __device__ __forceinline__ void own_rows_from_splits(const GemmDev& g, const CommDev& c, const CommCtx& x,
                                                      const int* counter, int mt, float* scratch) {
-    constexpr int kRows = 2;
-    constexpr int kGroup = 3;  // splits whose loads are in flight together (per row)
     const int t = threadIdx.x;
     const int threads = c.n / kVec;
     const bool active = t < threads;
@@ -148,6 +146,13 @@ __device__ __forceinline__ void own_rows_from_splits(const GemmDev& g, const Com
     }
     stamp(c, x, 2);
     stamp(c, x, 3);
+}
+
+template <int MODE>
+__device__ __forceinline__ void own_rows_from_splits(const GemmDev& g, const CommDev& c, const CommCtx& x,
+                                                     const int* counter, int mt, float* scratch) {
+    if (c.rows <= x.blocks) own_rows_from_splits<MODE, 1, 8>(g, c, x, counter, mt, scratch);
+    else own_rows_from_splits<MODE, 2, 3>(g, c, x, counter, mt, scratch);
 }
 
 // The early L2 prefetch of the rest of the weight slab pays for narrow tiles only; with 256-token tiles the stream is
