@@ -13,8 +13,6 @@ alone, for callers that hold GEMM2's input already quantised in the expert-major
 Nothing numeric runs in Python here: tensors are only laid out and handed to libdlmrt_b200.so.
 """
 
-from operator import is_
-
 import torch
 
 from .. import _lib
@@ -206,16 +204,14 @@ class FrontBuffers:
         self.act_codes = torch.zeros(count * rows, intermediate // 2, **u8)
         self.act_scales = torch.zeros(count * rows, intermediate // 16, **u8)
         self.down = Buffers(rows, hidden, top_k, device)
-        self.sources = ()  # the experts' tensors that `front` and `back` were filled in from
+        self.addresses = None  # of the experts' tensors that `front` and `back` were filled in from
         self.front = self.back = None
 
-    def fill(self, experts, sources, num_experts):
+    def fill(self, experts, addresses, num_experts):
         """The descriptors of both halves with everything in them that no call changes. Filling 40 fields anew was half of
         a small call's time on the host (27 us of three launches)."""
         f = DlmMoeFront()
-        w13, s13, g1, a2_inv = sources[:4]
-        f.w13_codes, f.w13_scales = w13.data_ptr(), s13.data_ptr()
-        f.g1, f.a2_inv = g1.data_ptr(), a2_inv.data_ptr()
+        f.w13_codes, f.w13_scales, f.g1, f.a2_inv = addresses[:4]
         f.ids, f.weights, f.counts, f.amap = (t.data_ptr() for t in (self.ids, self.weights, self.counts, self.amap))
         f.slot_codes, f.slot_scales = self.slot_codes.data_ptr(), self.slot_scales.data_ptr()
         f.act_codes, f.act_scales = self.act_codes.data_ptr(), self.act_scales.data_ptr()
@@ -224,7 +220,7 @@ class FrontBuffers:
         f.w13_tiled = 1
         self.back = descriptor(self.act_codes, self.act_scales, self.amap, self.counts, experts, self.ids, self.weights,
                                self.down, num_experts)
-        self.sources, self.front = sources, f
+        self.addresses, self.front = addresses, f
 
 
 # The experts' tensors whose addresses the descriptors of a FrontBuffers hold.
@@ -263,8 +259,9 @@ def trtllm_moe(x, packed, experts, out, num_experts, lo, intermediate, quantized
         b = cache[rows] = FrontBuffers(rows, hidden, intermediate, experts["w2"].shape[0], num_experts, packed.shape[1],
                                        x.device)
     sources = tuple(experts[key] for key in _SOURCES)
-    if not b.sources or not all(map(is_, sources, b.sources)) or b.front.e_total != num_experts:
-        b.fill(experts, sources, num_experts)
+    addresses = [t.data_ptr() for t in sources]
+    if addresses != b.addresses or b.front.e_total != num_experts:
+        b.fill(experts, addresses, num_experts)
     f = DlmMoeFront.from_buffer_copy(b.front)
     if quantized is None:
         f.x, f.a1_inv = x.data_ptr(), experts["a1_inv"].data_ptr()
