@@ -675,7 +675,7 @@ int dlm_moe_front_nvfp4(const DlmMoeFront* a, int pdl, dlm_stream_t stream) {
     d->aq_out = static_cast<uint8_t*>(a->act_codes), d->as_out = static_cast<uint8_t*>(a->act_scales);
     d->m = a->m, d->n = 2 * a->f, d->f = a->hidden, d->top_k = a->top_k, d->m_max = a->m_max;
     d->lo = a->lo, d->e_local = a->e_local, d->e_total = a->e_total;
-    d->f_out = a->f, d->act_kind = a->activation;
+    d->f_out = a->f, d->act_kind = a->activation, d->packed = a->packed;
     set_layout(d);
     p.fused = 0;
     return launch_moe_gate_up(p, info.sms, {s, true, false});  // always a dependent launch of the kernel above

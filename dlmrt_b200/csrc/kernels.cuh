@@ -69,6 +69,7 @@ struct alignas(64) MoeDev {
     const float* a2_inv;      // [e_local] 1 / (GEMM2 input scale): global scale of the activation's NVFP4 rounding
     uint8_t* aq_out;          // [e_local * m_max, f_out / 2] activation codes written into the expert-major slots
     uint8_t* as_out;          // [e_local * m_max, f_out / 16] their E4M3 scales (linear)
+    const int* packed;        // [m, top_k] expert << 16 | BF16 weight bits
     int f_out, act_kind;      // F; 0 = SwiGLU, 1 = GeGLU (tanh GELU)
 };
 

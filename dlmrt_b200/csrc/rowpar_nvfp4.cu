@@ -70,6 +70,7 @@ struct MoeSmem {
     uint32_t tmem_base;
     int n_active, epoch, gen, failed;
     int warp_count[8];
+    int counted[kMaxLocalExperts];  // GATE_UP: rows of each local expert
     float scratch[64];
     short active[kMaxEntries];  // expert | row block << 8
     short rows[kMaxEntries];    // rows of that block
@@ -323,13 +324,35 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
     if (warp == 2) tmem_alloc(&sm->tmem_base, kTmemCols);
     // The next kernel of the stream may be set up from now on (its blocks move in as this kernel's blocks leave).
     pdl_launch_dependents();
-    // Routing (counts, slots, activations) comes from the previous kernels of the stream: nothing of it may be read
-    // before they are complete.
-    pdl_wait();
+    if (GATE_UP) {
+        // The kernel in front of this one (moe_prepare_kernel) triggers only after it has itself waited for everything
+        // before it, so the packed top-k may be read already: the rows of each expert are counted from it here, and the
+        // weight stream starts while that kernel is still quantising rows into their slots. The roles that touch the
+        // slots wait for it. Four layers of 32 tokens, 256 experts: 274 us waiting first, 262 this way.
+        for (int e = threadIdx.x; e < kMaxLocalExperts; e += kMoeThreads) sm->counted[e] = 0;
+        __syncthreads();
+        const int pairs = g.m * g.top_k;
+        for (int first = threadIdx.x; first < pairs; first += 4 * kMoeThreads) {
+            int word[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (first + u * kMoeThreads < pairs) word[u] = __ldcg(g.packed + first + u * kMoeThreads);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int e = first + u * kMoeThreads < pairs ? (word[u] >> 16) - g.lo : -1;
+                if (e >= 0 && e < g.e_local) atomicAdd(&sm->counted[e], 1);
+            }
+        }
+        __syncthreads();
+    } else {
+        // Routing (counts, slots, activations) comes from the previous kernels of the stream: nothing of it may be read
+        // before they are complete.
+        pdl_wait();
+    }
     // Compact list of (expert, block of rows_cap rows) entries that have rows, in expert order.
     {
         const int e = threadIdx.x;
-        const int total_rows = e < g.e_local ? min(g.counts[g.lo + e], g.m_max) : 0;
+        const int total_rows = e < g.e_local ? min(GATE_UP ? sm->counted[e] : g.counts[g.lo + e], g.m_max) : 0;
         int early = 0;  // the invocation counters, fetched in the same round trip as the counts
         if (!GATE_UP) {
             if (threadIdx.x == 352 && p.fused) early = c.epochs[block];
@@ -422,6 +445,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
         const bool leader = elect_one();
         int buf = 0;
         uint32_t phase = 1;
+        if (GATE_UP) pdl_wait();  // the slots are filled by the kernel in front
         for (int entry = first_entry; entry <= last_entry; ++entry) {
             if (!mbar_wait_warp(&sm->a_empty[buf], phase, deadline)) {
                 if (leader) report(c.status, kErrTimeout, buf, kPhasePipeline, 5);
@@ -532,6 +556,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
         // group 1 the odd ones. What it needs from global memory (the expert's scale, the destination rows) changes with
         // the entry only.
         const int quarter = warp & 3, group = (warp - 4) >> 2;
+        if (GATE_UP) pdl_wait();  // the slots written below may still be read by the kernels before
         int entry = -1, cnt = 0, slot0 = 0;
         float g2 = 0.f, a2i = 0.f;
         int dest[kMaxRowsCap / 32];  // destination of row 32 q + lane
