@@ -194,7 +194,7 @@ class FrontBuffers:
     def __init__(self, rows, hidden, intermediate, count, num_experts, top_k, device):
         u8 = dict(device=device, dtype=torch.uint8)
         i32 = dict(device=device, dtype=torch.int32)
-        self.rows = rows
+        self.rows, self.top_k, self.num_experts = rows, top_k, num_experts
         self.ids = torch.zeros(rows, top_k, **i32)
         self.weights = torch.zeros(rows, top_k, device=device, dtype=torch.float32)
         self.counts = torch.zeros(num_experts, **i32)
@@ -207,7 +207,7 @@ class FrontBuffers:
         self.addresses = None  # of the experts' tensors that `front` and `back` were filled in from
         self.front = self.back = None
 
-    def fill(self, experts, addresses, num_experts):
+    def fill(self, experts, addresses):
         """The descriptors of both halves with everything in them that no call changes. Filling 40 fields anew was half of
         a small call's time on the host (27 us of three launches)."""
         f = DlmMoeFront()
@@ -215,12 +215,27 @@ class FrontBuffers:
         f.ids, f.weights, f.counts, f.amap = (t.data_ptr() for t in (self.ids, self.weights, self.counts, self.amap))
         f.slot_codes, f.slot_scales = self.slot_codes.data_ptr(), self.slot_scales.data_ptr()
         f.act_codes, f.act_scales = self.act_codes.data_ptr(), self.act_scales.data_ptr()
-        f.m, f.hidden, f.f, f.top_k, f.m_max = self.rows, experts["hidden"], experts["f"], self.ids.shape[1], self.rows
-        f.lo, f.e_local, f.e_total = experts["lo"], experts["w2"].shape[0], num_experts
+        f.m, f.hidden, f.f, f.top_k, f.m_max = self.rows, experts["hidden"], experts["f"], self.top_k, self.rows
+        f.lo, f.e_local, f.e_total = experts["lo"], experts["w2"].shape[0], self.num_experts
         f.w13_tiled = 1
         self.back = descriptor(self.act_codes, self.act_scales, self.amap, self.counts, experts, self.ids, self.weights,
-                               self.down, num_experts)
+                               self.down, self.num_experts)
         self.addresses, self.front = addresses, f
+
+
+def _front_buffers(experts, rows, top_k, num_experts, device):
+    """The layer's FrontBuffers for calls of this size, made on the first one: before any graph capture, as the reference
+    tunes. Nothing is ever replaced, because captured graphs hold the addresses. The buffers of a row count's first call
+    are found under the row count alone; `top_k` and `num_experts`, which size them too, are the same for all calls of
+    an ordinary program, and calls with other ones have buffers of their own."""
+    cache = experts.setdefault("_buffers", {})
+    key, b = rows, cache.get(rows)
+    if b is not None and (b.top_k != top_k or b.num_experts != num_experts):
+        key = rows, top_k, num_experts
+        b = cache.get(key)
+    if b is None:
+        b = cache[key] = FrontBuffers(rows, experts["hidden"], experts["f"], experts["w2"].shape[0], num_experts, top_k, device)
+    return b
 
 
 # The experts' tensors whose addresses the descriptors of a FrontBuffers hold.
@@ -253,21 +268,19 @@ def trtllm_moe(x, packed, experts, out, num_experts, lo, intermediate, quantized
     if experts["f"] != intermediate or experts["hidden"] != hidden:
         raise ValueError(f"experts are hidden {experts['hidden']}, intermediate {experts['f']}; the call says {hidden}, "
                          f"{intermediate}")
-    cache = experts.setdefault("_buffers", {})
-    b = cache.get(rows)
-    if b is None:  # first call with this row count: before any graph capture, as the reference tunes
-        b = cache[rows] = FrontBuffers(rows, hidden, intermediate, experts["w2"].shape[0], num_experts, packed.shape[1],
-                                       x.device)
+    if packed.shape[0] < rows:
+        raise ValueError(f"packed lists the experts of {packed.shape[0]} rows; the input has {rows}")
+    b = _front_buffers(experts, rows, packed.shape[1], num_experts, x.device)
     sources = tuple(experts[key] for key in _SOURCES)
     addresses = [t.data_ptr() for t in sources]
-    if addresses != b.addresses or b.front.e_total != num_experts:
-        b.fill(experts, addresses, num_experts)
+    if addresses != b.addresses:
+        b.fill(experts, addresses)
     f = DlmMoeFront.from_buffer_copy(b.front)
     if quantized is None:
         f.x, f.a1_inv = x.data_ptr(), experts["a1_inv"].data_ptr()
     else:
         f.xq, f.xs = x.data_ptr(), xs.data_ptr()
-    f.packed, f.top_k, f.activation = packed.data_ptr(), packed.shape[1], ACTIVATIONS[activation]
+    f.packed, f.activation = packed.data_ptr(), ACTIVATIONS[activation]
     code = _lib.lib().dlm_moe_front_nvfp4(f, 1, _lib.stream(x))
     if code:
         _lib.check(code, "trtllm_moe: front half")

@@ -207,3 +207,28 @@ def test_down_projection_is_deferred_into_the_reduction():
     torch.cuda.synchronize()
     g.check()
     assert_same_bits(bits(out), bits(plain), "fused vs unfused")
+
+
+def test_two_list_lengths_at_one_row_count():
+    """Calls of the same experts and row count with other top-k lengths must not share scratch sized for one of them:
+    each gives the bits of a first call on experts laid out afresh."""
+    from dlmrt_b200.quantization import nvfp4
+
+    prefix = "swiglu"
+    parts, e_total = golden_parts(prefix)
+    x = to_torch(G[f"{prefix}_x"]).cuda()
+    f = G[f"{prefix}_gate_packed"].shape[1]
+    g = torch.Generator().manual_seed(5)
+
+    def lists(top_k):
+        ids = torch.stack([torch.randperm(e_total, generator=g)[:top_k].sort().values for _ in range(x.shape[0])])
+        return nvfp4.pack(ids.int(), torch.rand(x.shape[0], top_k, generator=g)).cuda()
+
+    packed = [lists(top_k) for top_k in (2, 5, 2, 8)]
+    used = nvfp4.b200_experts(parts, 0, 0, e_total, "cuda")
+    for p in packed:
+        got, want = torch.empty_like(x), torch.empty_like(x)
+        nvfp4.trtllm_moe(x, p, used, got, e_total, 0, f, activation=prefix)
+        nvfp4.trtllm_moe(x, p, nvfp4.b200_experts(parts, 0, 0, e_total, "cuda"), want, e_total, 0, f, activation=prefix)
+        torch.cuda.synchronize()
+        assert_same_bits(bits(got), bits(want), f"top-{p.shape[1]}")
