@@ -143,6 +143,16 @@ def stream(tensor):
     return torch._C._cuda_getCurrentRawStream(device)
 
 
+def scratch(held, nbytes, device):
+    """Zero-initialised scratch of at least `nbytes` out of `held`, a list that belongs to one object. A larger buffer is
+    added when the newest is too small, and the older ones stay: graphs captured with them still write there. Sizes at
+    least double, so the old ones together are never larger than the newest."""
+    if not held or held[-1].numel() < nbytes:
+        with torch.inference_mode(False):  # shared by graphs captured in and out of inference mode
+            held.append(torch.zeros(max(nbytes, 2 * held[-1].numel()) if held else nbytes, device=device, dtype=torch.uint8))
+    return held[-1]
+
+
 def check(code, where):
     if code != OK:
         raise DlmError(code, where)

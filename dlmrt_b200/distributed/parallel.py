@@ -111,7 +111,7 @@ class Group:
         self._out_peers = {}
         self._last = {}      # per chain: the previous call's output buffer
         self._pending = {}   # partial data_ptr -> (linear, x): GEMMs deferred into the next reduction
-        self._workspaces = {}
+        self._workspaces = {}  # per chain: split-K scratch, see _lib.scratch
         self._gather = {}    # per key: slot addresses, invocation counters, multicast address of the slots
         self.stamps = 0      # device address of a [grid, 8] int64 buffer to record kernel phase times
         self._failed = False  # set by check() on a device time-out; the group must then be rebuilt
@@ -244,12 +244,7 @@ class Group:
 
     def workspace(self, chain, nbytes):
         """Split-K scratch of the fused GEMMs of one chain (FP32 partial tiles + tile counters), grown on demand."""
-        ws = self._workspaces.get(chain)
-        if ws is None or ws.numel() < nbytes:
-            with torch.inference_mode(False):
-                ws = torch.zeros(nbytes, device=self.device, dtype=torch.uint8)
-            self._workspaces[chain] = ws
-        return ws
+        return _lib.scratch(self._workspaces.setdefault(chain, []), nbytes, self.device)
 
     # -- launches ---------------------------------------------------------------------------------------------------
     def _call(self, rows, n, site, chain, mode, one_shot):

@@ -55,7 +55,7 @@ class Linear:
         self.group = group
         # Tiling of this layer's GEMM (tiles along the tokens, K splits): 0 = chosen by the library for each call.
         self.token_tiles, self.splits = token_tiles, splits
-        self._workspace = None
+        self._workspaces = []  # split-K scratch, see _lib.scratch
         self._plans = {}  # rows -> (a DlmGemm with everything filled in that no call changes, workspace bytes)
         _lib.lib()
 
@@ -83,10 +83,7 @@ class Linear:
         if x_step != 1 or out_step != 1:
             raise ValueError("x and out must have a contiguous last dimension")
         template, nbytes = self.plan(m)
-        workspace = self._workspace
-        if workspace is None or workspace.numel() < nbytes:
-            with torch.inference_mode(False):
-                workspace = self._workspace = torch.zeros(nbytes, device=x.device, dtype=torch.uint8)
+        workspace = _lib.scratch(self._workspaces, nbytes, x.device)
         g = DlmGemm.from_buffer_copy(template)
         self.describe(g)
         g.x, g.ldx = x.data_ptr(), ldx
