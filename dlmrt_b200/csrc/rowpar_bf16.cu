@@ -33,6 +33,7 @@ struct SmemLayout {
     uint32_t tmem_base;
     int epoch, gen, failed;  // epochs[block], gen[block] and status[0], fetched by a spare warp while the pipeline runs
     int seen[2];             // k-blocks each of two issuers has seen arrive (only kept on rings with an odd number of stages)
+    int stalled;             // a wait of this block ran out: it announces, pushes and stores nothing
     float scratch[64];
 };
 
@@ -64,7 +65,7 @@ __device__ __forceinline__ void own_rows_from_splits(const GemmDev& g, const Com
     uint4 wraw = make_uint4(0, 0, 0, 0);
     if (MODE != kReduce && active) wraw = *reinterpret_cast<const uint4*>(c.weight + col);
     int ready_tile = -1;  // rows are owned in increasing order, so token tiles are waited for in increasing order
-    bool ok = true;
+    bool ok = !x.dead;    // after a failure of this group no row is written any more, neither OUT nor the residual stream
     for (int r0 = x.block; r0 < c.rows; r0 += kRows * x.blocks) {
         size_t off[kRows];
         uint4 hraw[kRows];
@@ -234,7 +235,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
                 tma_load_2d(tiles + it * stage_bytes + kTileBytesW, &g.tm_x, &sm->full[it], (kb0 + it) * kBlockK,
                             token0, kEvictLast);
         }
-        if (leader) sm->seen[0] = sm->seen[1] = 0;
+        if (leader) sm->seen[0] = sm->seen[1] = sm->stalled = 0;
         __syncwarp();
     }
     if (warp == 2) tmem_alloc(&sm->tmem_base, cols * issuers);
@@ -310,7 +311,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
                         ok = __all_sync(0xFFFFFFFFu, ok);
                     }
                     if (!ok || !mbar_wait_warp(&sm->full[st], parity, pipeline_deadline)) {
-                        if (leader) report(c.status, kErrTimeout, st, kPhasePipeline, stalled(1, it));
+                        if (leader) {
+                            report(c.status, kErrTimeout, st, kPhasePipeline, stalled(1, it));
+                            sm->stalled = 1;  // the commit below completes acc_full all the same
+                        }
                         break;
                     }
                     if (guarded && leader) seen[who] = it + 1;
@@ -339,7 +343,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
         bool ok = true;
         if (iters > 0) {
             ok = mbar_wait(&sm->acc_full, 0, pipeline_deadline);
-            if (!ok) report(c.status, kErrTimeout, 0, kPhasePipeline, stalled(2, iters));
+            if (!ok) {
+                report(c.status, kErrTimeout, 0, kPhasePipeline, stalled(2, iters));
+                sm->stalled = 1;
+            }
             tcgen05_fence_after();
         }
         if (c.stamps && threadIdx.x == 128) c.stamps[block * kStampSlots + 4] = globaltimer();
@@ -396,7 +403,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
         if (threadIdx.x == 0) {
             for (int j = block; j < kMaxTiles; j += blocks) g.counters[((gen + 1) & 1) * kMaxTiles + j] = 0;
             __threadfence();  // after the block barrier: orders every thread's partial-tile stores before the announce
-            atomicAdd(g.counters + (gen & 1) * kMaxTiles + t, 1);
+            // A tile that never came out of the pipeline is not announced: its owners' waits run out in turn.
+            if (!sm->stalled) atomicAdd(g.counters + (gen & 1) * kMaxTiles + t, 1);
             for (int j = block; j < kEpochSlots; j += blocks) g.gen[j] = gen;
         }
     } else if (g.splits > 1) {
@@ -409,13 +417,14 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
         if (threadIdx.x == 0) {
             for (int j = block; j < kMaxTiles; j += blocks) g.counters[((gen + 1) & 1) * kMaxTiles + j] = 0;
             __threadfence();  // after the block barrier: orders every thread's partial-tile stores before the announce
-            atomicAdd(counter, 1);
+            if (!sm->stalled) atomicAdd(counter, 1);
             int seen;
             do {
                 asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
                 if (seen >= g.splits) break;
                 if (globaltimer() > pipeline_deadline) {
                     report(c.status, kErrTimeout, s, kPhasePipeline, 3 << 24);
+                    sm->stalled = 1;
                     break;
                 }
             } while (true);
@@ -423,7 +432,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
         }
         __syncthreads();
         const int tok_lo = static_cast<int>(static_cast<long long>(s) * mt / g.splits);
-        const int tok_hi = static_cast<int>(static_cast<long long>(s + 1) * mt / g.splits);
+        const int tok_hi = sm->stalled ? tok_lo : static_cast<int>(static_cast<long long>(s + 1) * mt / g.splits);
         const float* base = g.ws + static_cast<size_t>(tile) * g.splits * mt * kBlockF;
         const size_t split_stride = static_cast<size_t>(mt) * kBlockF;
         for (int v = threadIdx.x; v < (tok_hi - tok_lo) * (kBlockF / kVec); v += kFusedThreads) {
@@ -464,7 +473,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
         }
     } else {
         const uint4* staged = reinterpret_cast<const uint4*>(tiles);
-        for (int v = threadIdx.x; v < mt * (kBlockF / kVec); v += kFusedThreads) {
+        const int vecs = sm->stalled ? 0 : mt * (kBlockF / kVec);
+        for (int v = threadIdx.x; v < vecs; v += kFusedThreads) {
             const int token = v / (kBlockF / kVec), j = v % (kBlockF / kVec);
             const uint4 packed = staged[v];
             const int col = f * kBlockF + j * kVec;

@@ -69,6 +69,7 @@ struct MoeSmem {
     uint64_t acc_empty[2];
     uint32_t tmem_base;
     int n_active, epoch, gen, failed;
+    int stalled;  // a wait of this block ran out: it announces, pushes and stores nothing
     int warp_count[8];
     int counted[kMaxLocalExperts];  // GATE_UP: rows of each local expert
     float scratch[64];
@@ -318,6 +319,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
             mbar_init(&sm->acc_empty[i], 4);  // one arrival per epilogue warp of the buffer's group
         }
         fence_barrier_init();
+        sm->stalled = 0;
         if (!g.w_tiles) tma_prefetch_descriptor(&g.tm_w);
         tma_prefetch_descriptor(&g.tm_a);
     }
@@ -579,6 +581,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
             }
             if (!mbar_wait(&sm->acc_full[group], ((i - i0) >> 1) & 1, deadline)) {
                 report(c.status, kErrTimeout, 0, kPhasePipeline, 2);
+                sm->stalled = 1;
                 break;
             }
             tcgen05_fence_after();
@@ -627,7 +630,8 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
         if (threadIdx.x == 0) {
             if (block == 0) g.counters[((gen + 1) & 1) * kMaxTiles] = 0;
             __threadfence();  // after the block barrier: orders every thread's Y stores before the announce
-            atomicAdd(counter, 1);
+            // Rows that never came out of the pipeline are not announced: whoever combines them runs out of time in turn.
+            if (!sm->stalled) atomicAdd(counter, 1);
             // Only CTAs that have output rows to combine need the others' Y rows; polling is paced so that the
             // arrivals of the rest of the grid are not queued behind a storm of loads on the same word.
             while (block < g.m) {
@@ -636,6 +640,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
                 if (seen >= blocks) break;
                 if (globaltimer() > deadline) {
                     report(c.status, kErrTimeout, 0, kPhasePipeline, 3);
+                    sm->stalled = 1;
                     break;
                 }
                 __nanosleep(100);
@@ -648,12 +653,15 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
     // Combine: out[row] = bf16(sum over k in list order of w_k * y_k), experts of other ranks contribute 0 * 0.
     // With one rank the sum over ranks is the identity and the CTA that combines a row is also its owner (rows block,
     // block + blocks, ... in both roles), so the row is finished here and never travels through the receive slots.
+    // After a failure, of this launch or of an earlier one of the group, no row is written any more: neither the output
+    // nor the residual stream (x.dead is false in an unfused launch, and push_store looks at it itself).
     const bool local_rows = p.fused && c.world == 1;
-    if (local_rows) {
+    const bool write = !sm->stalled && !(local_rows && x.dead);
+    if (write && local_rows) {
         if (c.mode == kReduce) combine_and_finish<kReduce>(g, c, block, blocks, sm->scratch, first);
         else if (c.mode == kReduceNorm) combine_and_finish<kReduceNorm>(g, c, block, blocks, sm->scratch, first);
         else combine_and_finish<kReduceNormResidual>(g, c, block, blocks, sm->scratch, first);
-    } else {
+    } else if (write) {
         const int t = threadIdx.x, threads = g.n / kVec;
         for (int row = block; row < g.m; row += blocks) {
             if (t < threads) {

@@ -396,3 +396,49 @@ def test_one_rank_reduces_without_slots(rows, n, max_ctas):
             assert_norm_close(bits(out), want, f"call {i} mode {mode}")
         if mode == 2:
             assert_same_bits(bits(h), h_after[0], f"call {i}: residual stream")
+
+
+@pytest.mark.parametrize("path", ["reduce", "splits, one row a block", "splits, two rows a block", "one split", "experts"])
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_a_failed_one_rank_group_writes_nothing(path, mode):
+    """Once a wait of a group has run out, later launches write neither the output nor the residual stream until the host
+    has read the status, also where one rank finishes its rows without the receive slots. The failure is planted in the
+    status words; no wait runs out here."""
+    from dlmrt_b200 import _lib
+    from dlmrt_b200.distributed.parallel import Group
+    from dlmrt_b200.layers.linear import Linear
+
+    g = Group.local("cuda:0")
+    rows, n, k = (256 if "two" in path else 32), 2048, 1024
+    weight = randn_bf16(n, seed=1) if mode else None
+    h = randn_bf16(rows, n, seed=2) if mode == 2 else None
+    partial = g.partial("p", (rows, n))
+    if path == "reduce":
+        partial.copy_(randn_bf16(rows, n, seed=3))
+    elif path == "experts":
+        import test_moe_gpu
+
+        args = test_moe_gpu.device_args(test_moe_gpu.make_case(rows, n, 512, 8, 2, seed=4, exact=True), 0, 8)
+    else:
+        lin = Linear(randn_bf16(n, k, seed=5, std=0.02), group=g, token_tiles=1, splits=1 if "one split" in path else 3)
+        x = randn_bf16(rows, k, seed=6)
+
+    def call(site):
+        if path == "experts":
+            g.defer_experts(partial, args)
+        elif path != "reduce":
+            lin(x, out=partial)
+        return g.reduce(partial, site=site) if weight is None else g.reduce_norm(partial, h, weight, 1e-6, site=site)
+
+    assert bool((call("before").view(torch.int16) != -1).any())
+    torch.cuda.synchronize()
+    g.check()
+    g.status[0] = _lib.ERR_TIMEOUT
+    h_before = h.clone() if h is not None else None
+    out = call("after")
+    torch.cuda.synchronize()
+    assert bool((out.view(torch.int16) == -1).all()), "the output was written after a failure"
+    if h is not None:
+        assert torch.equal(h.view(torch.int16), h_before.view(torch.int16)), "the residual stream was written after a failure"
+    with pytest.raises(TimeoutError):
+        g.check()
