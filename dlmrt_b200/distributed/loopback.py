@@ -120,18 +120,8 @@ class LoopbackWorld:
         comms = (DlmComm * self.world)()
         outs = []
         for r, g in enumerate(self.groups):
-            out = g.symmetric(key, (self.world, *xs[r].shape), xs[r].dtype)
-            if key not in g._gather:
-                g.symmetric(key + ".slots", (3, self.world, nbytes // 2), armed=True)
-                epochs = torch.zeros(_lib.EPOCH_SLOTS, device=self.device, dtype=torch.int32)
-                g._gather[key] = list(g._handles[key + ".slots"].buffer_ptrs), epochs, 0
-            ptrs, epochs, _ = g._gather[key]
-            c = DlmComm()
-            c.rank, c.world = r, self.world
-            for s in range(self.world):
-                c.recv[s] = ptrs[s]
-            c.out, c.epochs, c.status = out.data_ptr(), epochs.data_ptr(), g.status.data_ptr()
-            c.timeout_ns, c.max_ctas = 500_000_000, g.max_ctas
+            c, out = g._gather_call(xs[r], nbytes, key)
+            c.timeout_ns, c.pdl = 500_000_000, 0
             comms[r] = c
             outs.append(out)
         ptrs = (C.c_void_p * self.world)(*[x.data_ptr() for x in xs])

@@ -112,7 +112,7 @@ class Group:
         self._last = {}      # per chain: the previous call's output buffer
         self._pending = {}   # partial data_ptr -> (linear, x): GEMMs deferred into the next reduction
         self._workspaces = {}  # per chain: split-K scratch, see _lib.scratch
-        self._gather = {}    # per key: slot addresses, invocation counters, multicast address of the slots
+        self._gather = {}    # per key: DlmComm template of its all-gathers
         self.stamps = 0      # device address of a [grid, 8] int64 buffer to record kernel phase times
         self._failed = False  # set by check() on a device time-out; the group must then be rebuilt
         self.status = torch.zeros(_lib.STATUS_WORDS, device=device, dtype=torch.int32)
@@ -416,6 +416,12 @@ class Group:
                              f"of 16 bytes, at most {_lib.GATHER_MAX_BYTES}; got {tuple(x.shape)} {x.dtype}")
         if self._failed:
             raise RuntimeError("this group reported a device time-out; build a new Group")
+        c, out = self._gather_call(x, nbytes, key)
+        _lib.check(_lib.lib().dlm_all_gather(x.data_ptr(), nbytes, c, _lib.stream(self.status)), f"all_gather {key}")
+        return out
+
+    def _gather_call(self, x, nbytes, key):
+        """The DlmComm of one all-gather and its output buffer; what every call of `key` has in common is filled in once."""
         out = self.symmetric(key, (self.world, *x.shape), x.dtype)
         template = self._gather.get(key)
         if template is None:
@@ -431,5 +437,4 @@ class Group:
             self._gather[key] = template
         c = DlmComm.from_buffer_copy(template)
         c.timeout_ns, c.pdl, c.max_ctas = TIMEOUT_NS, PDL, self.max_ctas
-        _lib.check(_lib.lib().dlm_all_gather(x.data_ptr(), nbytes, c, _lib.stream(self.status)), f"all_gather {key}")
-        return out
+        return c, out

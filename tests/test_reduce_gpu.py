@@ -442,3 +442,17 @@ def test_a_failed_one_rank_group_writes_nothing(path, mode):
         assert torch.equal(h.view(torch.int16), h_before.view(torch.int16)), "the residual stream was written after a failure"
     with pytest.raises(TimeoutError):
         g.check()
+
+
+def test_gathers_of_one_key_through_both_entry_points():
+    """A group's all-gathers of one key may go through the loopback launch and through the group itself, in any order."""
+    from dlmrt_b200.distributed.loopback import LoopbackWorld
+
+    for first_loopback in (True, False):
+        lw = LoopbackWorld(1)
+        for i in range(6):
+            x = torch.randn(32, 4, device="cuda")
+            out = lw.all_gather([x], "stats")[0] if (i % 2 == 0) == first_loopback else lw.groups[0].all_gather(x, "stats")
+            torch.cuda.synchronize()
+            lw.check()
+            assert torch.equal(out[0], x), f"call {i}"
