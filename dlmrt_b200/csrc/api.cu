@@ -1,5 +1,6 @@
 // extern "C" boundary of libdlmrt_b200.so (include/dlmrt_b200.h): argument checks, tensor-map construction, launch.
 // Mirrors the host checks of the reference's launch<> (dlmrt/ops/csrc/tp_comm.cu:282-287) as return codes.
+#include <cstdint>
 #include <cstring>
 
 #include "../../include/dlmrt_b200.h"
@@ -177,31 +178,25 @@ void choose_tiling(int m, int n, int k, int avail, int* tiles_out, int* splits_o
     }
 }
 
-// FP32 partial tiles of a GEMM whose K is split, as far as the library's own choice goes: kMaxSplits of every output tile,
-// or one tile of 128 features per SM where the output has so few that its K is split further.
-size_t partial_bytes(int m, int n) {
-    const size_t columns = static_cast<size_t>(kMaxSplits) * n, one_per_sm = static_cast<size_t>(148) * kBlockF;
-    return (columns > one_per_sm ? columns : one_per_sm) * m * sizeof(float);
-}
-
 // A plain GEMM of few output tiles and long K: kMaxSplits leave SMs idle (16 CTAs for 256 features), so choose_tiling's
 // pick is weighed against as many splits as there are SMs, half of them and so on. Beyond kMaxSplits every split costs
 // 0.2 us (the sum reads eight at a time, and fewer tokens are left for each CTA to sum). Measured, us with at most
 // kMaxSplits and beyond: 256 x 256 x 16384 14.3 and 11.8, 32 x 256 x 16384 13.5 and 10.0, 256 x 128 x 65536 40.5 and
 // 18.9; 64 x 512 x 4096 stays (7.7 with 8 splits, 7.9 with 9).
-void split_further(const DlmGemm* g, int avail, int* tiles, int* splits) {
-    const int feature_tiles = g->n / kBlockF, nkb = (g->k + kBlockK - 1) / kBlockK;
-    const double hbm = static_cast<double>(g->n) * g->k * 2 / 6.0e6;
+// `room`: bytes the workspace has for partial tiles.
+void split_further(int m, int n, int k, int64_t room, int avail, int* tiles, int* splits) {
+    const int feature_tiles = n / kBlockF, nkb = (k + kBlockK - 1) / kBlockK;
+    const double hbm = static_cast<double>(n) * k * 2 / 6.0e6;
     auto cost = [&](int t, int sp) {
-        const int mt = g->m / t, kb = (nkb + sp - 1) / sp;
+        const int mt = m / t, kb = (nkb + sp - 1) / sp;
         double us = kb * (0.24 + 0.0009 * mt);
         if (us < hbm) us = hbm;
         if (sp > 1) us += 2.8 + 0.019 * mt;
         return us + (sp > kMaxSplits ? 0.2 * (sp - kMaxSplits) : 0);
     };
-    const int64_t room = g->workspace_bytes - static_cast<int64_t>(kWorkspaceHeader), per_split = static_cast<int64_t>(g->m) * g->n * 4;
+    const int64_t per_split = static_cast<int64_t>(m) * n * 4;
     double best = cost(*tiles, *splits);
-    for (int t = 1; t <= 4 && g->m % (16 * t) == 0; t *= 2) {
+    for (int t = 1; t <= 4 && m % (16 * t) == 0; t *= 2) {
         for (int sp = avail / (feature_tiles * t); sp > kMaxSplits; sp /= 2) {
             if (sp > nkb || sp * per_split > room) continue;
             const double us = cost(t, sp);
@@ -236,7 +231,8 @@ int fill_gemm(GemmDev* d, const DlmGemm* g, int max_ctas, int sms, int* grid, in
         int t = 1, sp = 1;
         choose_tiling(g->m, g->n, g->k, avail, &t, &sp, owner_rows, single_rank);
         if (token_tiles == 0 && splits == 0) {
-            if (plain) split_further(g, avail, &t, &sp);
+            if (plain)
+                split_further(g->m, g->n, g->k, g->workspace_bytes - static_cast<int64_t>(kWorkspaceHeader), avail, &t, &sp);
             token_tiles = t;
             splits = sp;
         } else if (token_tiles == 0) {
@@ -752,10 +748,18 @@ int dlm_rowpar_bf16_loopback(const DlmGemm* gemm, const DlmComm* comm, int nrank
     return launch_rowpar_loopback(p, grid, nranks, {static_cast<cudaStream_t>(stream), false, true});
 }
 
+// Room for kMaxSplits partial tiles whatever K, or for as many as a plain GEMM of this shape splits its K into.
 size_t dlm_workspace_bytes(int m, int n, int k) {
-    (void)k;
     if (m <= 0 || n <= 0) return 0;
-    return kWorkspaceHeader + partial_bytes(m, n);
+    int tiles = 1, splits = kMaxSplits;
+    if (m >= 16 && m <= DLM_MAX_M && m % 16 == 0 && n % kBlockF == 0 && k >= kBlockK) {
+        DeviceInfo info;
+        const int sms = device_info(&info) == DLM_OK ? info.sms : 148;
+        choose_tiling(m, n, k, sms, &tiles, &splits);
+        split_further(m, n, k, INT64_MAX, sms, &tiles, &splits);
+        if (splits < kMaxSplits) splits = kMaxSplits;
+    }
+    return kWorkspaceHeader + static_cast<size_t>(splits) * m * n * sizeof(float);
 }
 
 int dlm_choose_tiling(int m, int n, int k, int max_ctas, int* token_tiles, int* splits) {

@@ -52,6 +52,17 @@ def test_strerror_and_sizes():
     assert lib.dlm_workspace_bytes(0, 2560, 64) == 0
 
 
+def test_workspace_follows_the_splits_a_shape_takes():
+    """Room for eight partial tiles, as an explicit request may ask for, and for more only where a plain GEMM of few
+    output tiles and long K is split further: a narrow layer with a short K does not pay for it."""
+    lib = _lib.lib()
+    for m, n, k in [(256, 128, 64), (256, 256, 1024), (16, 128, 512), (256, 2560, 4096), (32, 2048, 512), (64, 512, 4096)]:
+        assert lib.dlm_workspace_bytes(m, n, k) == 2048 + 8 * m * n * 4, (m, n, k)
+    for m, n, k in [(256, 128, 65536), (256, 256, 16384), (32, 256, 16384), (16, 128, 9472)]:
+        splits, rest = divmod(lib.dlm_workspace_bytes(m, n, k) - 2048, m * n * 4)
+        assert rest == 0 and 8 < splits <= 148 // (n // 128), (m, n, k, splits)
+
+
 def comm(**kw):
     c = DlmComm()
     c.rank, c.world, c.rows, c.n, c.mode = 0, 1, 32, 256, _lib.REDUCE
