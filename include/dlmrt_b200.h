@@ -301,10 +301,15 @@ DLM_API int dlm_all_gather(const void* x, int64_t bytes, const DlmComm* comm, dl
 DLM_API int dlm_all_gather_loopback(const void* const* x, int64_t bytes, const DlmComm* comm, int nranks,
                                     dlm_stream_t stream);
 
-/* Bytes of workspace (FP32 split-K partial tiles + tile counters) a GEMM of this shape needs. */
+/* Bytes of workspace (FP32 split-K partial tiles + tile counters) a GEMM of this shape needs: for 8 splits, or for as
+ * many as dlm_gemm_bf16 splits the K of this shape into. */
 DLM_API size_t dlm_workspace_bytes(int m, int n, int k);
 
-/* The (token tiles, K splits) the library would pick for this shape with `max_ctas` CTAs available (0 = all SMs). */
+/* The (token tiles, K splits) that the library's cost model picks for this shape among at most 8 splits, with `max_ctas`
+ * CTAs available (0 = all SMs); both are valid as explicit requests. dlm_gemm_bf16_noalloc runs with it, as far as its
+ * scratch goes. dlm_gemm_bf16 does too, except that an output of few tiles with a long K is split further when its
+ * workspace has dlm_workspace_bytes (which then has room for that number of splits). A GEMM in front of a reduction
+ * weighs the phase of the rows' owners as well and may run with another pick. */
 DLM_API int dlm_choose_tiling(int m, int n, int k, int max_ctas, int* token_tiles, int* splits);
 
 /* Copies the device status words to the host (synchronises `stream`) and clears them on the device. */

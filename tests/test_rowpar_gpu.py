@@ -58,15 +58,18 @@ def test_gemm_exact_on_integer_operands(m, n, k):
     assert_same_bits(bits(gemm(x, w)), want, f"gemm {m}x{n}x{k}")
 
 
-@pytest.mark.parametrize("m, n, k", [(16, 128, 9472), (256, 128, 20040), (32, 256, 16384), (144, 384, 6408), (80, 640, 8200),
-                                     (64, 128, 640)])
-def test_gemm_of_few_tiles_splits_k_further(m, n, k):
-    """Outputs of one to five feature tiles: up to one split per SM, K ragged (20040, 6408, 8200 are no multiples of a
-    k-block), as many splits as k-blocks (640 = 10), tokens that do not divide among the splits. Twice on the same
-    workspace, whose counters alternate; and with no room beyond eight splits."""
+@pytest.mark.parametrize("m, n, k, splits", [(16, 128, 9472, 18), (256, 128, 20040, 18), (32, 256, 16384, 18),
+                                             (144, 384, 6408, 12), (80, 640, 8200, 14), (16, 128, 1088, 9), (256, 128, 65536, 37),
+                                             (16, 128, 151936, 74)])
+def test_gemm_of_few_tiles_splits_k_further(m, n, k, splits):
+    """Outputs of one to five feature tiles: K split 9 to 74 ways (one split for every two SMs), ragged K (20040, 6408,
+    8200 are no multiples of a k-block), ranges of one or two k-blocks (1088 = 17 in 9 splits), tokens that do not divide
+    among the splits, fewer tokens than splits. Twice on the same workspace, whose counters alternate; and with no room
+    beyond eight splits. The number of splits is the one that the workspace has room for."""
     from dlmrt_b200 import _lib
     from dlmrt_b200._lib import DlmGemm
 
+    assert _lib.lib().dlm_workspace_bytes(m, n, k) == 2048 + splits * m * n * 4
     x, w = integer_case(m, n, k, seed=m + n + k)
     want = f32_to_bf16(rowpar.gemm_f32(bits(x), bits(w)))
     out = torch.empty(m, n, dtype=torch.bfloat16, device=x.device)
@@ -80,6 +83,8 @@ def test_gemm_of_few_tiles_splits_k_further(m, n, k):
             _lib.check(_lib.lib().dlm_gemm_bf16(C.byref(g), out.data_ptr(), n, 0, None), "gemm")
             torch.cuda.synchronize()
             assert_same_bits(bits(out), want, f"gemm {m}x{n}x{k}, workspace {nbytes}")
+            written = int(ws[2048:].view(torch.int32).view(-1, m * n).ne(0).any(1).sum())  # partial tiles the launch left
+            assert written == splits if nbytes > 2048 + 8 * m * n * 4 else written <= 8
 
 
 @pytest.mark.parametrize("m, n, k", SHAPES)
