@@ -689,7 +689,8 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
 
 template <int NR, bool GATE_UP>
 static int launch_impl(const MoeParams<NR>& p, dim3 grid, const LaunchOpts& o) {
-    const int smem = moe_smem_bytes(p.g[0]);
+    int smem = moe_smem_bytes(p.g[0]);
+    for (unsigned i = 1; i < grid.y; ++i) smem = max(smem, moe_smem_bytes(p.g[i]));  // emulated ranks may differ in f
     static bool raised[64] = {};
     cudaError_t err = cudaSuccess;
     int dev = 0;

@@ -207,3 +207,22 @@ def test_fused_residual_norm_after_the_experts(world):
     for r in range(world):
         assert_norm_close(bits(outs[r]), want, f"rank {r}")
         assert_same_bits(bits(hs[r]), h_after[r], f"residual of rank {r}")
+
+
+def test_emulated_ranks_of_different_intermediate_sizes():
+    """Ranks emulated in one launch have shared-memory layouts of their own (here 10 stages and larger row buffers, and 11
+    stages): the launch has to ask for the largest."""
+    from dlmrt_b200.distributed.loopback import LoopbackWorld
+    from dlmrt_b200.quantization import nvfp4
+
+    rows, hidden, e_total, top_k = 32, 512, 16, 4
+    cases = [make_case(rows, hidden, f, e_total, top_k, seed=17, exact=True) for f in (704, 512)]
+    assert np.array_equal(cases[0]["ids"], cases[1]["ids"])
+    keep = [device_args(case, r * 8, 8) for r, case in enumerate(cases)]
+    lw = LoopbackWorld(2)
+    outs = lw.moe([nvfp4.descriptor(**args) for args in keep], site="moe")
+    torch.cuda.synchronize()
+    lw.check()
+    want = red.reduce(np.stack([oracle_out(case, r * 8, 8)[0] for r, case in enumerate(cases)]))
+    for r, out in enumerate(outs):
+        assert_same_bits(bits(out), want, f"rank {r}")
