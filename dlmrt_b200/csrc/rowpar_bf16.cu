@@ -33,7 +33,6 @@ struct SmemLayout {
     uint32_t tmem_base;
     int epoch, gen, failed;  // epochs[block], gen[block] and status[0], fetched by a spare warp while the pipeline runs
     int seen[2];             // k-blocks each of two issuers has seen arrive (only kept on rings with an odd number of stages)
-    int stalled;             // a wait of this block ran out: it announces, pushes and stores nothing
     float scratch[64];
 };
 
@@ -235,7 +234,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
                 tma_load_2d(tiles + it * stage_bytes + kTileBytesW, &g.tm_x, &sm->full[it], (kb0 + it) * kBlockK,
                             token0, kEvictLast);
         }
-        if (leader) sm->seen[0] = sm->seen[1] = sm->stalled = 0;
+        if (leader) sm->seen[0] = sm->seen[1] = 0;
         __syncwarp();
     }
     if (warp == 2) tmem_alloc(&sm->tmem_base, cols * issuers);
@@ -251,6 +250,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
     // What a pipeline wait that ran out puts in the status' last word: who gave up (0 producer, 1 issuer, 2 epilogue,
     // 3 split-K rendezvous) and the k-block it was at.
     auto stalled = [](int who, int it) { return who << 24 | (it & 0xFFFF); };
+    bool bad = false;  // a wait of this thread ran out: its block announces, pushes and stores nothing
     if (warp == 0) {
         int st = pre == g.stages ? 0 : pre;
         uint32_t parity = 0;  // second lap of the ring waits for the first release of each stage
@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
                     if (!ok || !mbar_wait_warp(&sm->full[st], parity, pipeline_deadline)) {
                         if (leader) {
                             report(c.status, kErrTimeout, st, kPhasePipeline, stalled(1, it));
-                            sm->stalled = 1;  // the commit below completes acc_full all the same
+                            bad = true;  // the commit below completes acc_full all the same
                         }
                         break;
                     }
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
             ok = mbar_wait(&sm->acc_full, 0, pipeline_deadline);
             if (!ok) {
                 report(c.status, kErrTimeout, 0, kPhasePipeline, stalled(2, iters));
-                sm->stalled = 1;
+                bad = true;
             }
             tcgen05_fence_after();
         }
@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
         tcgen05_fence_before();
     }
     pdl_wait();
-    __syncthreads();
+    bad = __syncthreads_or(bad);
     if (warp == 2) {
         tcgen05_fence_after();
         tmem_dealloc(tmem, cols * issuers);
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
             for (int j = block; j < kMaxTiles; j += blocks) g.counters[((gen + 1) & 1) * kMaxTiles + j] = 0;
             __threadfence();  // after the block barrier: orders every thread's partial-tile stores before the announce
             // A tile that never came out of the pipeline is not announced: its owners' waits run out in turn.
-            if (!sm->stalled) atomicAdd(g.counters + (gen & 1) * kMaxTiles + t, 1);
+            if (!bad) atomicAdd(g.counters + (gen & 1) * kMaxTiles + t, 1);
             for (int j = block; j < kEpochSlots; j += blocks) g.gen[j] = gen;
         }
     } else if (g.splits > 1) {
@@ -417,22 +417,22 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
         if (threadIdx.x == 0) {
             for (int j = block; j < kMaxTiles; j += blocks) g.counters[((gen + 1) & 1) * kMaxTiles + j] = 0;
             __threadfence();  // after the block barrier: orders every thread's partial-tile stores before the announce
-            if (!sm->stalled) atomicAdd(counter, 1);
+            if (!bad) atomicAdd(counter, 1);
             int seen;
             do {
                 asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
                 if (seen >= g.splits) break;
                 if (globaltimer() > pipeline_deadline) {
                     report(c.status, kErrTimeout, s, kPhasePipeline, 3 << 24);
-                    sm->stalled = 1;
+                    bad = true;
                     break;
                 }
             } while (true);
             for (int j = block; j < kEpochSlots; j += blocks) g.gen[j] = gen;
         }
-        __syncthreads();
+        bad = __syncthreads_or(bad);
         const int tok_lo = static_cast<int>(static_cast<long long>(s) * mt / g.splits);
-        const int tok_hi = sm->stalled ? tok_lo : static_cast<int>(static_cast<long long>(s + 1) * mt / g.splits);
+        const int tok_hi = bad ? tok_lo : static_cast<int>(static_cast<long long>(s + 1) * mt / g.splits);
         const float* base = g.ws + static_cast<size_t>(tile) * g.splits * mt * kBlockF;
         const size_t split_stride = static_cast<size_t>(mt) * kBlockF;
         for (int v = threadIdx.x; v < (tok_hi - tok_lo) * (kBlockF / kVec); v += kFusedThreads) {
@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) rowpar_kernel(const __grid_c
         }
     } else {
         const uint4* staged = reinterpret_cast<const uint4*>(tiles);
-        const int vecs = sm->stalled ? 0 : mt * (kBlockF / kVec);
+        const int vecs = bad ? 0 : mt * (kBlockF / kVec);
         for (int v = threadIdx.x; v < vecs; v += kFusedThreads) {
             const int token = v / (kBlockF / kVec), j = v % (kBlockF / kVec);
             const uint4 packed = staged[v];

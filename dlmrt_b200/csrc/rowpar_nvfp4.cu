@@ -69,7 +69,6 @@ struct MoeSmem {
     uint64_t acc_empty[2];
     uint32_t tmem_base;
     int n_active, epoch, gen, failed;
-    int stalled;  // a wait of this block ran out: it announces, pushes and stores nothing
     int warp_count[8];
     int counted[kMaxLocalExperts];  // GATE_UP: rows of each local expert
     float scratch[64];
@@ -319,7 +318,6 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
             mbar_init(&sm->acc_empty[i], 4);  // one arrival per epilogue warp of the buffer's group
         }
         fence_barrier_init();
-        sm->stalled = 0;
         if (!g.w_tiles) tma_prefetch_descriptor(&g.tm_w);
         tma_prefetch_descriptor(&g.tm_a);
     }
@@ -408,6 +406,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
     const int last_entry = i1 > i0 ? (i1 - 1) / feature_tiles : first_entry - 1;
     const Cursor start{first_entry, i0 - first_entry * feature_tiles};
 
+    bool bad = false;  // a wait of this thread ran out: its block announces, pushes and stores nothing
     // Warps 0 to 2 run as whole warps on uniform values, one elected lane issuing (see uniform()).
     if (warp == 0) {
         const bool leader = elect_one();
@@ -581,7 +580,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
             }
             if (!mbar_wait(&sm->acc_full[group], ((i - i0) >> 1) & 1, deadline)) {
                 report(c.status, kErrTimeout, 0, kPhasePipeline, 2);
-                sm->stalled = 1;
+                bad = true;
                 break;
             }
             tcgen05_fence_after();
@@ -612,7 +611,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
     // Every Y row this CTA produced is written; announce it and wait for the rest of the grid (the combine reads rows
     // written by other CTAs). Counters are banked by launch generation as in the BF16 kernel.
     tcgen05_fence_before();
-    __syncthreads();
+    bad = __syncthreads_or(bad);
     if (c.stamps && threadIdx.x == 0) c.stamps[block * kStampSlots + 4] = globaltimer();
     if (warp == 2) {
         tcgen05_fence_after();
@@ -631,7 +630,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
             if (block == 0) g.counters[((gen + 1) & 1) * kMaxTiles] = 0;
             __threadfence();  // after the block barrier: orders every thread's Y stores before the announce
             // Rows that never came out of the pipeline are not announced: whoever combines them runs out of time in turn.
-            if (!sm->stalled) atomicAdd(counter, 1);
+            if (!bad) atomicAdd(counter, 1);
             // Only CTAs that have output rows to combine need the others' Y rows; polling is paced so that the
             // arrivals of the rest of the grid are not queued behind a storm of loads on the same word.
             while (block < g.m) {
@@ -640,14 +639,14 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
                 if (seen >= blocks) break;
                 if (globaltimer() > deadline) {
                     report(c.status, kErrTimeout, 0, kPhasePipeline, 3);
-                    sm->stalled = 1;
+                    bad = true;
                     break;
                 }
                 __nanosleep(100);
             }
             for (int j = block; j < kEpochSlots; j += blocks) g.gen[j] = gen;
         }
-        __syncthreads();
+        bad = __syncthreads_or(bad);
     }
     if (c.stamps && threadIdx.x == 0) c.stamps[block * kStampSlots + 5] = globaltimer();
     // Combine: out[row] = bf16(sum over k in list order of w_k * y_k), experts of other ranks contribute 0 * 0.
@@ -656,7 +655,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
     // After a failure, of this launch or of an earlier one of the group, no row is written any more: neither the output
     // nor the residual stream (x.dead is false in an unfused launch, and push_store looks at it itself).
     const bool local_rows = p.fused && c.world == 1;
-    const bool write = !sm->stalled && !(local_rows && x.dead);
+    const bool write = !bad && !(local_rows && x.dead);
     if (write && local_rows) {
         if (c.mode == kReduce) combine_and_finish<kReduce>(g, c, block, blocks, sm->scratch, first);
         else if (c.mode == kReduceNorm) combine_and_finish<kReduceNorm>(g, c, block, blocks, sm->scratch, first);
