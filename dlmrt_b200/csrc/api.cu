@@ -555,7 +555,7 @@ static int make_map_u8(CUtensorMap* map, const void* base, long long rows, int r
 
 static void set_layout(MoeDev* d) {
     const MoeLayout layout = moe_layout(d->f, d->m_max, d->m * d->top_k / d->e_total);
-    d->rows_cap = layout.rows_cap, d->buffers = layout.buffers, d->stages = layout.stages;
+    d->rows_cap = layout.rows_cap, d->buffers = layout.buffers, d->stages = layout.stages, d->resident = layout.resident;
 }
 
 static int fill_moe(MoeDev* d, const DlmMoe* m) {

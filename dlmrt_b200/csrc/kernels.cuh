@@ -64,7 +64,7 @@ struct alignas(64) MoeDev {
     __nv_bfloat16* out;       // plain (unfused) output [m, n]
     long long ldo;
     int m, n, f, top_k, m_max, lo, e_local, e_total;
-    int stages, rows_cap, buffers;  // shared memory: see moe_layout
+    int stages, rows_cap, buffers, resident;  // shared and tensor memory: see moe_layout
     // GEMM1 (gate / up) only: n = 2F interleaved weight rows, f = hidden, g2 = the GEMM1 alpha g1
     const float* a2_inv;      // [e_local] 1 / (GEMM2 input scale): global scale of the activation's NVFP4 rounding
     uint8_t* aq_out;          // [e_local * m_max, f_out / 2] activation codes written into the expert-major slots
@@ -124,6 +124,7 @@ int launch_moe_prepare(const PrepareDev& p, const LaunchOpts& o);
 int launch_route_packed(const RouteDev& p, const LaunchOpts& o);
 struct MoeLayout {
     int rows_cap, buffers, stages;  // rows of one entry, buffers for an entry's rows, stages of the weight ring
+    bool resident;                  // an entry's row scales stay in tensor memory
 };
 MoeLayout moe_layout(int k, int m_max, int mean_rows);
 int rowpar_smem_bytes(int m, int stages);

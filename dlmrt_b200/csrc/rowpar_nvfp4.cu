@@ -18,8 +18,8 @@
 //            its 2 KB of pre-interleaved 128 x 4 scale atoms (one bulk copy)
 //   warp 2   TMA, once per entry: its activation rows, all of K (boxes of 8 rows x 128 bytes)
 //   warp 3   once per entry: the rows' linear E4M3 scales, rewritten into scale atoms
-//   warp 1   per entry: tcgen05.cp the rows' scale atoms into tensor memory, where they stay for all its items (as long
-//            as K leaves room); per k-block: tcgen05.cp W2's atoms, then up to four
+//   warp 1   per entry: tcgen05.cp the rows' scale atoms into tensor memory, where they stay for all its items (where they
+//            fit, else again per k-block); per k-block: tcgen05.cp W2's atoms, then up to four
 //            tcgen05.mma.kind::mxf4nvf4.block_scale (K = 64) into the FP32 accumulator
 //   warps 4-11  two groups of four, one accumulator buffer each, alternate items: tcgen05.ld, times g2, BF16, scatter
 //            rows to Y[pair] through the expert's slot map
@@ -50,11 +50,12 @@ constexpr int kAtom = 512;             // one 128-row x 4-scale atom
 constexpr int kStepsPerBlock = 4;      // K = 64 instructions per 256-element k-block
 constexpr int kStageBytes = kCodeTileW + kStepsPerBlock * kAtom;  // 18 KB: a k-block's codes and scale atoms
 constexpr int kMaxRowsCap = 128;       // rows of one entry: the MMA's N
-// Tensor memory: two 128-column accumulators, two rotating sets of W2 scale columns (a k-block's copies need not wait for
-// the previous k-block's MMAs to finish reading theirs), and the entry's row scales: four columns per K = 64 step for as
-// many steps as fit (kSfbSteps), else two rotating sets like W2's.
-constexpr int kTmemAcc = 0, kTmemSfa = 256, kTmemSfb = 288, kTmemCols = 512;
-constexpr int kSfbSteps = (kTmemCols - kTmemSfb) / 4;
+// Tensor memory: two accumulators of rows_cap columns, then the scales of the MMAs' operands, four columns per K = 64 step.
+// Nothing orders a scale copy behind MMAs issued before it that still read the columns it overwrites (copy before MMA is
+// an ordered pair, MMA before copy is not), so every set of columns belongs to the shared memory it is copied from and
+// is overwritten only after that has been refilled, which waits for those MMAs: W2's scales have a set per ring stage,
+// the entry's row scales all of its steps per row buffer (`resident`) or, where these do not fit, a set per stage too.
+constexpr int kTmemCols = 512, kScaleCols = 4 * kStepsPerBlock;
 constexpr int kMaxLocalExperts = 256;
 constexpr int kMaxEntries = 2 * kMaxLocalExperts;  // one per active expert + one per 16 rows of 4096 pairs at most
 constexpr int kMoeStages = 12;
@@ -92,11 +93,11 @@ MoeLayout moe_layout(int k, int m_max, int mean_rows) {
     int most = (m_max + 15) / 16 * 16;
     if (most > kMaxRowsCap) most = kMaxRowsCap;
     auto stages_of = [&](int cap, int buffers) { return (kMoeSmemBudget - buffers * entry_bytes(cap, k)) / kStageBytes; };
-    MoeLayout best{16, 1, 1};
+    MoeLayout best{16, 1, 1, false};
     for (int want = 6; want >= 4; --want) {
         for (int cap = most; cap >= 16; cap -= 16) {
             if (stages_of(cap, 2) < want) continue;
-            best = {cap, 2, stages_of(cap, 2)};
+            best = {cap, 2, stages_of(cap, 2), false};
             break;
         }
         if (best.buffers == 2 && (best.rows_cap >= 32 || best.rows_cap == most)) break;
@@ -104,11 +105,20 @@ MoeLayout moe_layout(int k, int m_max, int mean_rows) {
     if (best.buffers == 1 || mean_rows > best.rows_cap) {
         for (int cap = most; cap > best.rows_cap || (best.buffers == 1 && cap >= 16); cap -= 16) {
             if (stages_of(cap, 1) < (cap == 16 ? 1 : 4)) continue;
-            best = {cap, 1, stages_of(cap, 1)};
+            best = {cap, 1, stages_of(cap, 1), false};
             break;
         }
     }
     if (best.stages > kMoeStages) best.stages = kMoeStages;
+    auto tmem_cols = [&](int stages, bool resident) {
+        const int rows = resident ? best.buffers * (k / 64) * 4 : stages * kScaleCols;
+        return 2 * best.rows_cap + stages * kScaleCols + rows;
+    };
+    // A stage less, out of six or more, costs less than copying the row scales again for every item.
+    if (best.stages > 5 && tmem_cols(best.stages, true) > kTmemCols && tmem_cols(best.stages - 1, true) <= kTmemCols)
+        --best.stages;
+    best.resident = tmem_cols(best.stages, true) <= kTmemCols;
+    while (!best.resident && tmem_cols(best.stages, false) > kTmemCols) --best.stages;
     return best;
 }
 
@@ -477,18 +487,19 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
         }
         __syncwarp();
     } else if (warp == 1) {
-        // One lane feeds the tensor pipe, so everything it issues executes in that order: scale copies into columns
-        // that earlier MMAs read need no wait.
+        // One lane feeds the tensor pipe.
         const bool leader = elect_one();
         const uint64_t desc_hi = umma_desc_k128(tiles) & 0xFFFFFFFF00000000ull;     // swizzled operand tiles
         const uint64_t sf_hi = utccp_desc(tiles) & 0xFFFFFFFF00000000ull;           // scale atoms
         auto operand = [&](uint32_t address) { return desc_hi | ((address & 0x3FFFF) >> 4); };
         auto atom = [&](uint32_t address) { return sf_hi | ((address & 0x3FFFF) >> 4); };
         const uint32_t ring = smem_u32(tiles), scales = smem_u32(ring_scales), rows0 = smem_u32(entry_rows);
-        const bool resident = steps <= kSfbSteps;  // the entry's row scales stay in tensor memory
-        int st = 0, set = 0, buf = -1;
+        // Columns of the scales: W2's by ring stage, the entry's rows by row buffer and step, or by ring stage.
+        const uint32_t tmem_sfa = tmem + 2 * g.rows_cap, tmem_sfb = tmem_sfa + g.stages * kScaleCols;
+        const bool resident = g.resident;
+        int st = 0, buf = -1;
         uint32_t phase = 0, a_phase = 1;
-        uint32_t rows = 0, idesc = 0;
+        uint32_t rows = 0, row_scales = 0, idesc = 0;
         bool alive = true;
         Cursor at = start;
         for (int i = i0; i < i1 && alive; ++i, at.next(feature_tiles)) {
@@ -504,10 +515,11 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
                 fence_proxy_async();  // the scale atoms were written through the generic proxy
                 tcgen05_fence_after();
                 rows = rows0 + buf * rows_bytes;
+                row_scales = tmem_sfb + buf * steps * 4;
                 idesc = umma_idesc_nvfp4(kBlockF, (uniform(static_cast<int>(sm->rows[at.entry])) + 15) & ~15);
                 if (resident && leader)
                     for (int s2 = 0; s2 < steps; ++s2)
-                        utccp_128x4(tmem + kTmemSfb + 4 * s2, atom(rows + nkb * row_tile + s2 * kAtom));
+                        utccp_128x4(row_scales + 4 * s2, atom(rows + nkb * row_tile + s2 * kAtom));
             }
             // The accumulator buffer must have been read out by the epilogue of two items ago.
             if (item >= 2 && !mbar_wait_warp(&sm->acc_empty[acc_buf], ((item >> 1) - 1) & 1, deadline)) {
@@ -515,7 +527,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
                 break;
             }
             tcgen05_fence_after();
-            const uint32_t acc = tmem + kTmemAcc + acc_buf * kMaxRowsCap;
+            const uint32_t acc = tmem + acc_buf * g.rows_cap;
             for (int kb = 0; kb < nkb; ++kb) {
                 if (!mbar_wait_warp(&sm->full[st], phase, deadline)) {
                     if (leader) report(c.status, kErrTimeout, st, kPhasePipeline, 1);
@@ -525,8 +537,8 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
                 tcgen05_fence_after();
                 const uint64_t dw = operand(ring + st * kCodeTileW), da = operand(rows + kb * row_tile);
                 const uint64_t fa = atom(scales + st * kStepsPerBlock * kAtom);
-                const uint32_t sfa = tmem + kTmemSfa + set * 4 * kStepsPerBlock;
-                const uint32_t sfb = tmem + kTmemSfb + 4 * kStepsPerBlock * (resident ? kb : set);
+                const uint32_t sfa = tmem_sfa + st * kScaleCols;
+                const uint32_t sfb = resident ? row_scales + kb * kScaleCols : tmem_sfb + st * kScaleCols;
                 const int nsteps = min(kStepsPerBlock, steps - kb * kStepsPerBlock);
                 if (leader) {
                     if (!resident) {
@@ -546,7 +558,6 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
                     }
                     umma_commit(&sm->empty[st]);
                 }
-                set ^= 1;
                 if (++st == g.stages) st = 0, phase ^= 1;
             }
             if (alive && leader) umma_commit(&sm->acc_full[acc_buf]);
@@ -585,7 +596,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
             }
             tcgen05_fence_after();
             const int col = at.ft * kBlockF + quarter * 32 + lane;
-            const uint32_t acc = tmem + kTmemAcc + group * kMaxRowsCap + (static_cast<uint32_t>(quarter * 32) << 16);
+            const uint32_t acc = tmem + group * g.rows_cap + (static_cast<uint32_t>(quarter * 32) << 16);
 #pragma unroll
             for (int chunk = 0; chunk < kMaxRowsCap / 16; ++chunk) {
                 if (chunk * 16 >= cnt) break;

@@ -232,3 +232,78 @@ def test_two_list_lengths_at_one_row_count():
         nvfp4.trtllm_moe(x, p, nvfp4.b200_experts(parts, 0, 0, e_total, "cuda"), want, e_total, 0, f, activation=prefix)
         torch.cuda.synchronize()
         assert_same_bits(bits(got), bits(want), f"top-{p.shape[1]}")
+
+
+def front_half(experts, x, packed, num_experts, activation):
+    """The front half alone (dlm_moe_front_nvfp4), on the scratch that `trtllm_moe` uses: also for hidden sizes that only
+    this half takes."""
+    from dlmrt_b200 import _lib
+    from dlmrt_b200._lib import DlmMoeFront
+    from dlmrt_b200.quantization import nvfp4
+
+    b = nvfp4._front_buffers(experts, x.shape[0], packed.shape[1], num_experts, x.device)
+    b.fill(experts, [experts[key].data_ptr() for key in nvfp4._SOURCES])
+    f = DlmMoeFront.from_buffer_copy(b.front)
+    f.x, f.a1_inv, f.packed = x.data_ptr(), experts["a1_inv"].data_ptr(), packed.data_ptr()
+    f.activation = nvfp4.ACTIVATIONS[activation]
+    _lib.check(_lib.lib().dlm_moe_front_nvfp4(f, 1, torch.cuda.current_stream().cuda_stream), "front half")
+    return b
+
+
+@pytest.mark.parametrize("rows, hidden, f, e_total, top_k, hot, activation", [
+    (256, 2048, 192, 8, 4, False, "swiglu"),   # more than 384 pairs to count, experts of several row blocks
+    (130, 2816, 64, 4, 2, True, "geglu"),      # one expert has every row: blocks of 80 rows, the last one ragged
+    (37, 2048, 512, 40, 4, False, "swiglu"),   # many short entries: several entries and items per CTA
+    (256, 256, 704, 16, 8, False, "geglu"),    # one k-block; several 16-row chunks per entry
+    (7, 2816, 128, 8, 3, False, "swiglu"),     # the 16-row layout
+    (256, 3072, 128, 8, 7, False, "swiglu"),   # one row buffer; 1792 pairs
+    (33, 3328, 128, 8, 2, False, "swiglu"),    # row scales copied per k-block
+    (256, 4096, 64, 4, 2, True, "swiglu"),     # K = 4096: one row buffer, and
+    (24, 4096, 64, 8, 2, False, "geglu"),      # two of 16 rows
+    (256, 6144, 64, 4, 2, True, "swiglu"),
+    (256, 8192, 64, 4, 3, False, "swiglu"),    # the longest K
+    (9, 8192, 128, 8, 2, False, "geglu"),
+])
+def test_gate_up_beyond_one_tile(rows, hidden, f, e_total, top_k, hot, activation):
+    """GEMM1 + activation + re-quantisation on several k-blocks, items per CTA, 16-row chunks and row blocks per expert, in
+    every layout that K forces on it; twice on the same scratch. Weights with power-of-two scales, so that the dots are
+    exact and only the approximate exponentials and reciprocals are left to differ by a step now and then."""
+    from dlmrt_b200.quantization import nvfp4
+
+    rng = np.random.default_rng(rows + hidden + f)
+    if hot:  # expert 0 is on every token's list
+        ids = np.stack([np.concatenate([[0], 1 + np.sort(rng.permutation(e_total - 1)[:top_k - 1])]) for _ in range(rows)])
+    else:
+        ids = np.stack([np.sort(rng.permutation(e_total)[:top_k]) for _ in range(rows)])
+    ids = ids.astype(np.int32)
+    pow2 = np.array([0x28, 0x30, 0x38, 0x40], dtype=np.uint8)  # E4M3 0.25, 0.5, 1, 2
+    codes, scales, parts = {}, {}, {}
+    for proj, n, k in (("gate", f, hidden), ("up", f, hidden), ("down", hidden, f)):
+        codes[proj] = rng.integers(0, 256, (e_total, n, k // 2), dtype=np.uint8)
+        scales[proj] = pow2[rng.integers(0, 4, (e_total, n, k // 16))]
+        for e in range(e_total):
+            parts[0, e, proj, "weight"] = torch.from_numpy(codes[proj][e])
+            parts[0, e, proj, "weight_scale"] = torch.from_numpy(scales[proj][e])
+            parts[0, e, proj, "weight_scale_2"] = torch.tensor(0.5 / hidden ** 0.5)
+            parts[0, e, proj, "input_scale"] = torch.tensor(2.0 ** -6 if proj != "down" else 2.0 ** -5)
+    experts = nvfp4.b200_experts(parts, 0, 0, e_total, "cuda")
+    x = to_torch(f32_to_bf16(rng.standard_normal((rows, hidden)).astype(np.float32))).cuda()
+    packed = torch.from_numpy(onv.pack_topk(ids, np.full(ids.shape, 0.5, dtype=np.float32))).cuda()
+    for _ in range(2):
+        b = front_half(experts, x, packed, e_total, activation)
+    torch.cuda.synchronize()
+    amap, counts = onv.route_slots(ids, e_total)
+    assert np.array_equal(b.counts.cpu().numpy(), counts)
+    slot_codes, slot_scales = b.slot_codes.cpu().numpy(), b.slot_scales.cpu().numpy()
+    got_codes, got_scales = b.act_codes.cpu().numpy(), b.act_scales.cpu().numpy()
+    g1 = experts["g1"].cpu().numpy()
+    want_codes, want_scales = np.zeros_like(got_codes), np.zeros_like(got_scales)
+    used = np.concatenate([np.arange(e * rows, e * rows + counts[e]) for e in range(e_total)])
+    for e in range(e_total):
+        if counts[e]:
+            sl = slice(e * rows, e * rows + counts[e])
+            want_codes[sl], want_scales[sl], act = onv.expert_gate_up(slot_codes[sl], slot_scales[sl], codes["gate"][e],
+                                                                      scales["gate"][e], codes["up"][e], scales["up"][e], g1[e],
+                                                                      np.float32(32), activation)
+            assert 0.05 < np.abs(act).mean() < 50  # the case is in the range that the scales can express
+    codes_close(got_codes[used], got_scales[used], want_codes[used], want_scales[used], "re-quantised activations")

@@ -226,3 +226,21 @@ def test_emulated_ranks_of_different_intermediate_sizes():
     want = red.reduce(np.stack([oracle_out(case, r * 8, 8)[0] for r, case in enumerate(cases)]))
     for r, out in enumerate(outs):
         assert_same_bits(bits(out), want, f"rank {r}")
+
+
+@pytest.mark.parametrize("rows, f, e_total, top_k, hot", [
+    (48, 2048, 6, 2, True),      # two row buffers of 32 rows, scales resident; a popular expert takes several row blocks
+    (16, 2816, 6, 2, False),     # two buffers of 16 rows; a ring stage given up so that the scales stay resident
+    (40, 3328, 4, 2, True),      # two buffers, scales copied per k-block
+    (256, 1024, 4, 3, True),     # one buffer of 128 rows, scales resident
+    (256, 3584, 4, 2, True),     # one buffer of 64 rows
+    (130, 3648, 4, 2, True),     # a last k-block of one step, several row blocks that no expert fills
+    (256, 4096, 4, 2, True),     # one buffer of 48 rows, scales copied per k-block
+    (37, 4096, 16, 2, False),    # two buffers of 16 rows, scales copied per k-block
+])
+def test_long_k_layouts_match_bit_for_bit(rows, f, e_total, top_k, hot):
+    """The layouts that shared and tensor memory force on longer K: fewer rows per block, one row buffer instead of two, row
+    scales that do not stay in tensor memory. Several items per CTA and several row blocks per expert."""
+    case = make_case(rows, 3072, f, e_total, top_k, seed=rows + f, exact=True, hot=hot)
+    want, _ = oracle_out(case, 0, e_total)
+    assert_same_bits(run_single(case), want, f"{rows} rows, f {f}")
