@@ -123,7 +123,7 @@ int launch_moe_gate_up(const MoeParams<1>& p, int grid, const LaunchOpts& o);
 int launch_moe_prepare(const PrepareDev& p, const LaunchOpts& o);
 int launch_route_packed(const RouteDev& p, const LaunchOpts& o);
 struct MoeLayout {
-    int rows_cap, buffers, stages;  // rows of one entry, buffers for an entry's rows, stages of the weight ring
+    int rows_cap, buffers, stages;  // rows of one entry, buffers for an entry's rows (0: streamed), stages of the ring
     bool resident;                  // an entry's row scales stay in tensor memory
 };
 MoeLayout moe_layout(int k, int m_max, int mean_rows);

@@ -23,6 +23,7 @@
 //            tcgen05.mma.kind::mxf4nvf4.block_scale (K = 64) into the FP32 accumulator
 //   warps 4-11  two groups of four, one accumulator buffer each, alternate items: tcgen05.ld, times g2, BF16, scatter
 //            rows to Y[pair] through the expert's slot map
+// (GEMM1 with a very long K streams the rows with the weights instead, see moe_layout.)
 // The kernel is bound by the HBM weight stream if nothing else holds it up, and what held it up was the chain behind each
 // k-block: one thread issuing eight scale copies, four MMAs and a commit (the commit alone waits ~340 ns behind eight
 // copies), and small copies of activation rows and scales repeated for every item. Rows kept per entry halve the scale
@@ -82,6 +83,9 @@ __host__ __device__ int entry_bytes(int rows_cap, int k) {
     return (k + 255) / 256 * rows_cap * 128 + (k / 64 + 1) / 2 * (2 * kAtom);  // a multiple of 1 KB
 }
 
+// The same for one k-block of the rows, as a ring stage holds it where rows are streamed with the weights.
+__host__ __device__ int row_stage_bytes(int rows_cap) { return rows_cap * 128 + kStepsPerBlock * kAtom; }
+
 }  // namespace
 
 // Picks rows_cap, the number of row buffers and the ring's stages for experts of `k` inputs and at most `m_max` rows, of
@@ -89,11 +93,16 @@ __host__ __device__ int entry_bytes(int rows_cap, int k) {
 // stages (108 KB in flight per SM cover HBM's latency at full rate), four at least. More rows per entry mean fewer
 // passes over an expert's weights (the later ones come out of L2), so the largest cap that leaves the ring its stages is
 // taken; where experts have many more rows than that on average, one larger buffer beats two small ones.
+// Where K is so long that one buffer holds 16 rows only (above 6400), rows are not kept at all but streamed: each ring
+// stage brings the entry's rows of its k-block along with the weights, `most` of them, again for every item. GEMM1 of two
+// layers with 1024 features, us with 16 rows kept and streamed: K = 8192, 64 experts of 32 rows 424 and 269, 8 of 256
+// 321 and 155, 64 of one 143 and 143; K = 6656, 128 of 8 303 and 314. Up to 6400, where 32 rows or more are kept, neither
+// is better everywhere: K = 6144 233 and 213, 156 and 128, but 156 and 167 with 16 experts of 128 rows.
 MoeLayout moe_layout(int k, int m_max, int mean_rows) {
     int most = (m_max + 15) / 16 * 16;
     if (most > kMaxRowsCap) most = kMaxRowsCap;
     auto stages_of = [&](int cap, int buffers) { return (kMoeSmemBudget - buffers * entry_bytes(cap, k)) / kStageBytes; };
-    MoeLayout best{16, 1, 1, false};
+    MoeLayout best{0, 0, 0, false};
     for (int want = 6; want >= 4; --want) {
         for (int cap = most; cap >= 16; cap -= 16) {
             if (stages_of(cap, 2) < want) continue;
@@ -102,28 +111,32 @@ MoeLayout moe_layout(int k, int m_max, int mean_rows) {
         }
         if (best.buffers == 2 && (best.rows_cap >= 32 || best.rows_cap == most)) break;
     }
-    if (best.buffers == 1 || mean_rows > best.rows_cap) {
-        for (int cap = most; cap > best.rows_cap || (best.buffers == 1 && cap >= 16); cap -= 16) {
-            if (stages_of(cap, 1) < (cap == 16 ? 1 : 4)) continue;
+    if (best.buffers == 0 || mean_rows > best.rows_cap) {
+        for (int cap = most; cap > best.rows_cap; cap -= 16) {
+            if (stages_of(cap, 1) < 4) continue;
             best = {cap, 1, stages_of(cap, 1), false};
             break;
         }
     }
+    if (best.buffers < 2 && best.rows_cap < 32 && best.rows_cap < most)
+        best = {most, 0, kMoeSmemBudget / (kStageBytes + row_stage_bytes(most)), false};
     if (best.stages > kMoeStages) best.stages = kMoeStages;
     auto tmem_cols = [&](int stages, bool resident) {
         const int rows = resident ? best.buffers * (k / 64) * 4 : stages * kScaleCols;
         return 2 * best.rows_cap + stages * kScaleCols + rows;
     };
     // A stage less, out of six or more, costs less than copying the row scales again for every item.
-    if (best.stages > 5 && tmem_cols(best.stages, true) > kTmemCols && tmem_cols(best.stages - 1, true) <= kTmemCols)
+    if (best.buffers > 0 && best.stages > 5 && tmem_cols(best.stages, true) > kTmemCols &&
+        tmem_cols(best.stages - 1, true) <= kTmemCols)
         --best.stages;
-    best.resident = tmem_cols(best.stages, true) <= kTmemCols;
+    best.resident = best.buffers > 0 && tmem_cols(best.stages, true) <= kTmemCols;
     while (!best.resident && tmem_cols(best.stages, false) > kTmemCols) --best.stages;
     return best;
 }
 
 static int moe_smem_bytes(const MoeDev& d) {
-    return d.stages * kStageBytes + d.buffers * entry_bytes(d.rows_cap, d.f) + static_cast<int>(sizeof(MoeSmem)) + 1024;
+    const int rows = d.buffers > 0 ? d.buffers * entry_bytes(d.rows_cap, d.f) : d.stages * row_stage_bytes(d.rows_cap);
+    return d.stages * kStageBytes + rows + static_cast<int>(sizeof(MoeSmem)) + 1024;
 }
 
 // A token's expert list for the combine step, eight entries at a time: local expert index (or -1) and routing weight.
@@ -293,7 +306,8 @@ __device__ __forceinline__ void requantise_chunk(const MoeDev& g, const uint32_t
     }
 }
 
-template <int NR, bool GATE_UP>
+// STREAMED: rows come with the weights, k-block by k-block (GEMM1 only: the down-projection takes no K that long).
+template <int NR, bool GATE_UP, bool STREAMED>
 __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_constant__ MoeParams<NR> p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const int slot = NR == 1 ? 0 : static_cast<int>(blockIdx.y);
@@ -308,17 +322,17 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
     const int nkb = (steps + kStepsPerBlock - 1) / kStepsPerBlock;
     const int scale_row = g.f / 16;              // bytes of scales per activation row
     const int row_tile = g.rows_cap * 128;       // bytes of one k-block of an entry's rows
-    const int rows_bytes = entry_bytes(g.rows_cap, g.f);
+    const int rows_bytes = STREAMED ? row_stage_bytes(g.rows_cap) : entry_bytes(g.rows_cap, g.f);
 
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     // The ring's codes, then its scale atoms, then the entries' rows: everything the MMAs read swizzled is 1 KB aligned.
     uint8_t* ring_scales = tiles + g.stages * kCodeTileW;
     uint8_t* entry_rows = tiles + g.stages * kStageBytes;
-    MoeSmem* sm = reinterpret_cast<MoeSmem*>(entry_rows + g.buffers * rows_bytes);
+    MoeSmem* sm = reinterpret_cast<MoeSmem*>(entry_rows + (STREAMED ? g.stages : g.buffers) * rows_bytes);
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < g.stages; ++i) {
-            mbar_init(&sm->full[i], 1);
+            mbar_init(&sm->full[i], STREAMED ? 34 : 1);  // the weights' expect_tx arrival (and the rows', as in a_full)
             mbar_init(&sm->empty[i], 1);
         }
         for (int i = 0; i < 2; ++i) {
@@ -452,38 +466,64 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
     } else if (warp == 2 || warp == 3) {
         // The entries' rows: codes by TMA (warp 2, one thread), scales by asynchronous copies straight into the atoms
         // (warp 3): atom byte (r % 32) * 16 + (r / 32) * 4 + j of step s holds scale 4 s + j of row r (< 128). A buffer is
-        // refilled once the MMAs of the entry it held have completed.
+        // refilled once the MMAs of the entry it held have completed. Streamed rows go into the ring's stages instead.
         const bool leader = elect_one();
-        int buf = 0;
-        uint32_t phase = 1;
         if (GATE_UP) pdl_wait();  // the slots are filled by the kernel in front
-        for (int entry = first_entry; entry <= last_entry; ++entry) {
-            if (!mbar_wait_warp(&sm->a_empty[buf], phase, deadline)) {
-                if (leader) report(c.status, kErrTimeout, buf, kPhasePipeline, 5);
-                break;
-            }
+        // K-blocks [kb0, kb0 + kbs) of an entry's rows into `codes` and `atoms`, announced on `bar`.
+        auto fetch = [&](int entry, int kb0, int kbs, uint8_t* codes, uint8_t* atoms, uint64_t* bar) {
             const int what = uniform(static_cast<int>(sm->active[entry])), cnt = uniform(static_cast<int>(sm->rows[entry]));
             const int row0 = (what & 0xFF) * g.m_max + (what >> 8) * g.rows_cap;  // first slot of the entry
-            uint8_t* rows = entry_rows + buf * rows_bytes;
             if (warp == 2) {
                 const int boxes = (cnt + kBoxRows - 1) / kBoxRows;
                 if (leader) {
-                    mbar_expect_tx(&sm->a_full[buf], static_cast<uint32_t>(nkb * boxes * kBoxRows * 128));
-                    for (int kb = 0; kb < nkb; ++kb)
+                    mbar_expect_tx(bar, static_cast<uint32_t>(kbs * boxes * kBoxRows * 128));
+                    for (int kb = 0; kb < kbs; ++kb)
                         for (int b = 0; b < boxes; ++b)
-                            tma_load_2d(rows + kb * row_tile + b * kBoxRows * 128, &g.tm_a, &sm->a_full[buf], kb * 128,
+                            tma_load_2d(codes + kb * row_tile + b * kBoxRows * 128, &g.tm_a, bar, (kb0 + kb) * 128,
                                         row0 + b * kBoxRows, kEvictLast);
                 }
             } else {
-                uint8_t* atoms = rows + nkb * row_tile;
-                for (int r = 0; r < cnt; ++r) {
-                    const uint8_t* src = g.a_scales + static_cast<size_t>(row0 + r) * scale_row;
-                    uint8_t* dst = atoms + (r % 32) * 16 + (r / 32) * 4;
-                    for (int s2 = lane; s2 < steps; s2 += 32) cp_async_4(dst + s2 * kAtom, src + s2 * 4);
+                const int step0 = kb0 * kStepsPerBlock, count = min(steps - step0, kbs * kStepsPerBlock);
+                const uint8_t* from = g.a_scales + static_cast<size_t>(row0) * scale_row + step0 * 4;
+                auto copy = [&](int r, int s2) {
+                    cp_async_4(atoms + s2 * kAtom + (r % 32) * 16 + (r / 32) * 4, from + static_cast<size_t>(r) * scale_row + s2 * 4);
+                };
+                if (STREAMED) {
+                    for (int r = lane; r < cnt; r += 32)
+                        for (int s2 = 0; s2 < count; ++s2) copy(r, s2);
+                } else {
+                    for (int r = 0; r < cnt; ++r)
+                        for (int s2 = lane; s2 < count; s2 += 32) copy(r, s2);
                 }
-                cp_async_arrive(&sm->a_full[buf]);
+                cp_async_arrive(bar);
             }
-            if (++buf == g.buffers) buf = 0, phase ^= 1;
+        };
+        int at_ring = 0;
+        uint32_t phase = 1;
+        if (STREAMED) {
+            Cursor at = start;
+            for (int i = i0; i < i1; ++i, at.next(feature_tiles)) {
+                for (int kb = 0; kb < nkb; ++kb) {
+                    if (!mbar_wait_warp(&sm->empty[at_ring], phase, deadline)) {
+                        if (leader) report(c.status, kErrTimeout, at_ring, kPhasePipeline, 5);
+                        i = i1;
+                        break;
+                    }
+                    uint8_t* rows = entry_rows + at_ring * rows_bytes;
+                    fetch(at.entry, kb, 1, rows, rows + row_tile, &sm->full[at_ring]);
+                    if (++at_ring == g.stages) at_ring = 0, phase ^= 1;
+                }
+            }
+        } else {
+            for (int entry = first_entry; entry <= last_entry; ++entry) {
+                if (!mbar_wait_warp(&sm->a_empty[at_ring], phase, deadline)) {
+                    if (leader) report(c.status, kErrTimeout, at_ring, kPhasePipeline, 5);
+                    break;
+                }
+                uint8_t* rows = entry_rows + at_ring * rows_bytes;
+                fetch(entry, 0, nkb, rows, rows + nkb * row_tile, &sm->a_full[at_ring]);
+                if (++at_ring == g.buffers) at_ring = 0, phase ^= 1;
+            }
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -504,7 +544,9 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
         Cursor at = start;
         for (int i = i0; i < i1 && alive; ++i, at.next(feature_tiles)) {
             const int item = i - i0, acc_buf = item & 1;
-            if (item == 0 || at.ft == 0) {  // a new entry
+            if (item == 0 || at.ft == 0)  // a new entry
+                idesc = umma_idesc_nvfp4(kBlockF, (uniform(static_cast<int>(sm->rows[at.entry])) + 15) & ~15);
+            if (!STREAMED && (item == 0 || at.ft == 0)) {
                 if (leader && buf >= 0) umma_commit(&sm->a_empty[buf]);
                 if (++buf == g.buffers) buf = 0;
                 if (buf == 0) a_phase ^= 1;
@@ -516,7 +558,6 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
                 tcgen05_fence_after();
                 rows = rows0 + buf * rows_bytes;
                 row_scales = tmem_sfb + buf * steps * 4;
-                idesc = umma_idesc_nvfp4(kBlockF, (uniform(static_cast<int>(sm->rows[at.entry])) + 15) & ~15);
                 if (resident && leader)
                     for (int s2 = 0; s2 < steps; ++s2)
                         utccp_128x4(row_scales + 4 * s2, atom(rows + nkb * row_tile + s2 * kAtom));
@@ -534,15 +575,17 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
                     alive = false;
                     break;
                 }
+                if (STREAMED) fence_proxy_async();  // as for the entry's scale atoms above
                 tcgen05_fence_after();
-                const uint64_t dw = operand(ring + st * kCodeTileW), da = operand(rows + kb * row_tile);
+                const uint32_t row_codes = STREAMED ? rows0 + st * rows_bytes : rows + kb * row_tile;
+                const uint64_t dw = operand(ring + st * kCodeTileW), da = operand(row_codes);
                 const uint64_t fa = atom(scales + st * kStepsPerBlock * kAtom);
                 const uint32_t sfa = tmem_sfa + st * kScaleCols;
                 const uint32_t sfb = resident ? row_scales + kb * kScaleCols : tmem_sfb + st * kScaleCols;
                 const int nsteps = min(kStepsPerBlock, steps - kb * kStepsPerBlock);
                 if (leader) {
                     if (!resident) {
-                        const uint64_t fb = atom(rows + nkb * row_tile + kb * kStepsPerBlock * kAtom);
+                        const uint64_t fb = atom(STREAMED ? row_codes + row_tile : rows + nkb * row_tile + kb * kStepsPerBlock * kAtom);
                         for (int s2 = 0; s2 < nsteps; ++s2) utccp_128x4(sfb + 4 * s2, fb + s2 * (kAtom >> 4));
                     }
                     if (nsteps == kStepsPerBlock) {
@@ -697,7 +740,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
     }
 }
 
-template <int NR, bool GATE_UP>
+template <int NR, bool GATE_UP, bool STREAMED = false>
 static int launch_impl(const MoeParams<NR>& p, dim3 grid, const LaunchOpts& o) {
     int smem = moe_smem_bytes(p.g[0]);
     for (unsigned i = 1; i < grid.y; ++i) smem = max(smem, moe_smem_bytes(p.g[i]));  // emulated ranks may differ in f
@@ -706,7 +749,7 @@ static int launch_impl(const MoeParams<NR>& p, dim3 grid, const LaunchOpts& o) {
     int dev = 0;
     (void)cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !raised[dev]) {
-        err = cudaFuncSetAttribute(moe_kernel<NR, GATE_UP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        err = cudaFuncSetAttribute(moe_kernel<NR, GATE_UP, STREAMED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    kMoeSmemBudget + static_cast<int>(sizeof(MoeSmem)) + 1024);
         raised[dev] = err == cudaSuccess;
     }
@@ -730,7 +773,7 @@ static int launch_impl(const MoeParams<NR>& p, dim3 grid, const LaunchOpts& o) {
         }
         config.attrs = attrs;
         config.numAttrs = n;
-        err = cudaLaunchKernelEx(&config, moe_kernel<NR, GATE_UP>, p);
+        err = cudaLaunchKernelEx(&config, moe_kernel<NR, GATE_UP, STREAMED>, p);
     }
     if (err != cudaSuccess) {
         g_last_cuda_error = static_cast<int>(err);
@@ -743,7 +786,9 @@ static int launch_impl(const MoeParams<NR>& p, dim3 grid, const LaunchOpts& o) {
 
 int launch_moe(const MoeParams<1>& p, int grid, const LaunchOpts& o) { return launch_impl<1, false>(p, dim3(grid), o); }
 
-int launch_moe_gate_up(const MoeParams<1>& p, int grid, const LaunchOpts& o) { return launch_impl<1, true>(p, dim3(grid), o); }
+int launch_moe_gate_up(const MoeParams<1>& p, int grid, const LaunchOpts& o) {
+    return p.g[0].buffers > 0 ? launch_impl<1, true>(p, dim3(grid), o) : launch_impl<1, true, true>(p, dim3(grid), o);
+}
 
 int launch_moe_loopback(const MoeParams<kMaxWorld>& p, int grid, int nranks, const LaunchOpts& o) {
     return launch_impl<kMaxWorld, false>(p, dim3(grid, nranks), o);

@@ -261,7 +261,9 @@ def front_half(experts, x, packed, num_experts, activation):
     (256, 4096, 64, 4, 2, True, "swiglu"),     # K = 4096: one row buffer, and
     (24, 4096, 64, 8, 2, False, "geglu"),      # two of 16 rows
     (256, 6144, 64, 4, 2, True, "swiglu"),
-    (256, 8192, 64, 4, 3, False, "swiglu"),    # the longest K
+    (48, 6400, 64, 4, 2, True, "geglu"),       # one row buffer of 32 rows, the longest K that keeps the rows
+    (40, 6656, 64, 4, 2, True, "swiglu"),      # rows streamed with the weights, 48 of them
+    (256, 8192, 64, 4, 3, False, "swiglu"),    # and 128, at the longest K; experts of two row blocks
     (9, 8192, 128, 8, 2, False, "geglu"),
 ])
 def test_gate_up_beyond_one_tile(rows, hidden, f, e_total, top_k, hot, activation):
