@@ -144,12 +144,11 @@ def stream(tensor):
 
 
 def scratch(held, nbytes, device):
-    """Zero-initialised scratch of at least `nbytes` out of `held`, a list that belongs to one object. A larger buffer is
-    added when the newest is too small, and the older ones stay: graphs captured with them still write there. Sizes at
-    least double, so the old ones together are never larger than the newest."""
-    if not held or held[-1].numel() < nbytes:
-        with torch.inference_mode(False):  # shared by graphs captured in and out of inference mode
-            held.append(torch.zeros(max(nbytes, 2 * held[-1].numel()) if held else nbytes, device=device, dtype=torch.uint8))
+    """Adds zero-initialised scratch of at least `nbytes` to `held`, a list that belongs to one object and whose buffers
+    are all too small. The older ones stay: graphs captured with them still write there. Sizes at least double, so the
+    old ones together are never larger than the newest."""
+    with torch.inference_mode(False):  # shared by graphs captured in and out of inference mode
+        held.append(torch.zeros(max(nbytes, 2 * held[-1].numel()) if held else nbytes, device=device, dtype=torch.uint8))
     return held[-1]
 
 

@@ -244,7 +244,11 @@ class Group:
 
     def workspace(self, chain, nbytes):
         """Split-K scratch of the fused GEMMs of one chain (FP32 partial tiles + tile counters), grown on demand."""
-        return _lib.scratch(self._workspaces.setdefault(chain, []), nbytes, self.device)
+        held = self._workspaces.get(chain)
+        if held is None or held[-1].numel() < nbytes:
+            held = self._workspaces.setdefault(chain, [])
+            _lib.scratch(held, nbytes, self.device)
+        return held[-1]
 
     # -- launches ---------------------------------------------------------------------------------------------------
     def _call(self, rows, n, site, chain, mode, one_shot):

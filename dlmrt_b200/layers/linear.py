@@ -55,7 +55,7 @@ class Linear:
         self.group = group
         # Tiling of this layer's GEMM (tiles along the tokens, K splits): 0 = chosen by the library for each call.
         self.token_tiles, self.splits = token_tiles, splits
-        self._workspaces = []  # split-K scratch, see _lib.scratch
+        self._workspace, self._workspaces = None, []  # split-K scratch: the newest, and all (see _lib.scratch)
         self._plans = {}  # rows -> (a DlmGemm with everything filled in that no call changes, workspace bytes)
         _lib.lib()
 
@@ -83,7 +83,9 @@ class Linear:
         if x_step != 1 or out_step != 1:
             raise ValueError("x and out must have a contiguous last dimension")
         template, nbytes = self.plan(m)
-        workspace = _lib.scratch(self._workspaces, nbytes, x.device)
+        workspace = self._workspace
+        if workspace is None or workspace.numel() < nbytes:
+            workspace = self._workspace = _lib.scratch(self._workspaces, nbytes, x.device)
         g = DlmGemm.from_buffer_copy(template)
         self.describe(g)
         g.x, g.ldx = x.data_ptr(), ldx
