@@ -95,9 +95,10 @@ __host__ __device__ int row_stage_bytes(int rows_cap) { return rows_cap * 128 + 
 // taken; where experts have many more rows than that on average, one larger buffer beats two small ones.
 // Where K is so long that one buffer holds 16 rows only (above 6400), rows are not kept at all but streamed: each ring
 // stage brings the entry's rows of its k-block along with the weights, `most` of them, again for every item. GEMM1 of two
-// layers with 1024 features, us with 16 rows kept and streamed: K = 8192, 64 experts of 32 rows 424 and 269, 8 of 256
-// 321 and 155, 64 of one 143 and 143; K = 6656, 128 of 8 303 and 314. Up to 6400, where 32 rows or more are kept, neither
-// is better everywhere: K = 6144 233 and 213, 156 and 128, but 156 and 167 with 16 experts of 128 rows.
+// layers with 1024 features, us with 16 rows kept and streamed: K = 8192, 64 experts of 32 rows 424 and 234, 8 of 256
+// 325 and 133, 64 of one 143 and 143; K = 6656, 128 of 8 303 and 311. Up to 6400 32 rows or more are kept: K = 4096, 64
+// experts of 32 rows 124 and 156, 16 of 128 96 and 128, 8 of 256 96 and 102; K = 6144 the same three 227 and 213, 149 and
+// 167, 147 and 128.
 MoeLayout moe_layout(int k, int m_max, int mean_rows) {
     int most = (m_max + 15) / 16 * 16;
     if (most > kMaxRowsCap) most = kMaxRowsCap;
@@ -485,15 +486,16 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_kernel(const __grid_consta
             } else {
                 const int step0 = kb0 * kStepsPerBlock, count = min(steps - step0, kbs * kStepsPerBlock);
                 const uint8_t* from = g.a_scales + static_cast<size_t>(row0) * scale_row + step0 * 4;
-                auto copy = [&](int r, int s2) {
-                    cp_async_4(atoms + s2 * kAtom + (r % 32) * 16 + (r / 32) * 4, from + static_cast<size_t>(r) * scale_row + s2 * 4);
-                };
-                if (STREAMED) {
-                    for (int r = lane; r < cnt; r += 32)
-                        for (int s2 = 0; s2 < count; ++s2) copy(r, s2);
-                } else {
-                    for (int r = 0; r < cnt; ++r)
-                        for (int s2 = lane; s2 < count; s2 += 32) copy(r, s2);
+                // A warp copies 2^lg rows of 32 / 2^lg steps at a time. The steps of one row all go to one bank (atoms are
+                // 512 bytes apart), so as many rows as there are share an instruction. With one row per instruction, 128
+                // rows of K = 2048 took longer than their codes: 8 experts of 134 rows, whole call, 54 us and 36 this way;
+                // 8 of 256 at hidden 2816 99 and 60; four layers of 256 experts under Zipf routing 215 and 196.
+                const int lg = min(5, 32 - __clz(cnt - 1));
+                for (int r = lane & ((1 << lg) - 1); r < cnt; r += 1 << lg) {
+                    const uint8_t* src = from + static_cast<size_t>(r) * scale_row;
+                    uint8_t* dst = atoms + (r % 32) * 16 + (r / 32) * 4;
+#pragma unroll 4
+                    for (int s2 = lane >> lg; s2 < count; s2 += 32 >> lg) cp_async_4(dst + s2 * kAtom, src + s2 * 4);
                 }
                 cp_async_arrive(bar);
             }
