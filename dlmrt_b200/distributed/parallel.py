@@ -11,7 +11,9 @@ discipline and error behaviour, so model code written against it runs unchanged.
     ranks' receive slots and reduces them (`Group.flush(partial)` materialises the partial if something else wants
     to read it);
   * NCCL is used only to create the process group torch symmetric memory rendezvouses over, as in the reference
-    (parallel.py:42-43,73); on a single GPU a `Group.local` (world 1) runs the same kernels over ordinary buffers.
+    (parallel.py:42-43,73); on a single GPU a `Group.local` (world 1) makes the same calls over ordinary buffers, of
+    which only an unsplit projection goes through the receive slots: the other reductions of one rank finish their rows
+    where they are.
 
 One process per GPU runs the same program; every reduction returns bitwise-identical values on all ranks.
 """
@@ -120,7 +122,7 @@ class Group:
 
     @classmethod
     def local(cls, device):
-        """A world-1 group on one GPU: same kernels, receive slots and output buffers in local memory."""
+        """A world-1 group on one GPU: same calls, with receive slots and output buffers in local memory."""
         return cls(torch.device(device), rank=0, world=1, allocator=LocalAllocator(torch.device(device)))
 
     def symmetric(self, key, shape, dtype=torch.bfloat16, armed=False):
